@@ -2,9 +2,9 @@
 //
 // Per tree level (see mf_plan.cu):
 //   k_small   : fronts with nj <= kSmallMax.  One CTA holds the whole frontal
-//               matrix in shared memory: load the assembled panel, extend-add
-//               the children's update matrices, partial LDL^T/Cholesky of the
-//               first nn columns, write panel + update matrix.  This fuses
+//               matrix: load the assembled panel, extend-add the children's
+//               update matrices, partial LDL^T/Cholesky of the first nn
+//               columns, write panel + update matrix.  This fuses
 //               chol_loop_snd!/chol_loop_nod! (cholesky.jl:434-692) for the
 //               many tiny fronts of a maximal-supernode tree.
 //   k_ea      : extend-add for larger fronts, one CTA per (front, 16 parent
@@ -148,176 +148,442 @@ __global__ void k_panel32_to_dl(const Front* __restrict__ fronts, const RefFront
 // (or 64 x 64 diagonal block), which is then factored again in FP64.
 constexpr double kRescueSmall = 1e-5;
 constexpr double kRescueGrowth = 1e7;
-constexpr int kSmallKids = 32;  // children whose records k_small fetches up front
+constexpr int kSmallKids = 16;  // children whose records k_small fetches up front
 
-// One small front held in shared memory as TC: load the assembled panel, add
-// the children (in the reference's reverse order), factor the first nn
-// columns right-looking.  Returns the first rejected pivot (front-local) or
-// -1; with `check`, *flag is set when a pivot is small or grown (see above).
-// Uniform across the block.
-template <typename TC, typename T, int LDLT>
-__device__ int small_front(TC* F, const Front& f, const Front* __restrict__ fronts,
-                           const int32_t* __restrict__ reltgt, const int32_t* __restrict__ chdtgt,
-                           const T* __restrict__ P, const T* __restrict__ M, const double* __restrict__ signs,
-                           bool check, int* flag, Reg reg) {
-    const int nn = f.nn, na = f.na, nj = nn + na, ld = f.ldp;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const T* Pj = P + f.poff;
-    // the children's records (first kSmallKids, in the order they are added),
-    // fetched at once beside the panel load instead of one dependent pair of
-    // loads per child
-    __shared__ int kid_na[kSmallKids], kid_lm[kSmallKids], kid_sep0[kSmallKids];
-    __shared__ int64_t kid_moff[kSmallKids];
-    const int nch = f.chd1 - f.chd0;
-    for (int q = tid; q < min(nch, kSmallKids); q += nt) {
-        const Front fc = fronts[chdtgt[f.chd1 - 1 - q]];
-        kid_na[q] = fc.na;
-        kid_lm[q] = fc.ldm;
-        kid_sep0[q] = fc.sep0;
-        kid_moff[q] = fc.moff;
+// The reciprocal ik that scales the column of an accepted pivot p: 1 / sqrt(p)
+// for Cholesky, 1 / p for LDLt.  The chain of dependent pivots waits for it, so
+// it takes the shortest sequence of full accuracy: in double CUDA's rsqrt (at
+// most 1 ulp off, what the rounded square root and the rounded division after
+// it reach together); in float the hardware's approximation and one
+// Newton-Raphson step (for y^-2 = p or y^-1 = p), dropped by a select where
+// the step's products leave the exponent range.  The stored diagonal entry
+// (sqrt(p), or p) is formed beside the chain.
+template <int LDLT>
+__device__ __forceinline__ float pivot_recip(float p) {
+    float y;
+    if (LDLT) {
+        asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(p));
+        const float z = fmaf(y, fmaf(-p, y, 1.0f), y);
+        return fabsf(y) > 1e-36f && fabsf(y) < 1e36f ? z : y;
     }
-    for (int i = tid; i < nj * nn; i += nt) {
-        int r = i % nj, c = i / nj;
-        F[i] = (TC)Pj[r + (int64_t)c * ld];
-    }
-    for (int i = tid; i < nj * na; i += nt) F[nj * nn + i] = TC(0);
-    __syncthreads();
-    // extend-add, children popped in reverse (cholesky.jl:506-514)
-    for (int q = 0; q < nch; ++q) {
-        int ma, lm, sep0;
-        int64_t moff;
-        if (q < kSmallKids) {
-            ma = kid_na[q], lm = kid_lm[q], sep0 = kid_sep0[q], moff = kid_moff[q];
-        } else {
-            const Front fc = fronts[chdtgt[f.chd1 - 1 - q]];
-            ma = fc.na, lm = fc.ldm, sep0 = fc.sep0, moff = fc.moff;
-        }
-        const int32_t* rel = reltgt + sep0;
-        const T* Mc = M + moff;
-        for (int i = tid; i < ma * ma; i += nt) {
-            int a = i % ma, b = i / ma;
-            if (a >= b) F[rel[a] + rel[b] * nj] += (TC)Mc[a + b * lm];
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(p));
+    const float z = fmaf(0.5f * y, fmaf(-(p * y), y, 1.0f), y);
+    return p < 1e36f ? z : y;
+}
+template <int LDLT>
+__device__ __forceinline__ double pivot_recip(double p) {
+    return LDLT ? 1.0 / p : rsqrt(p);
+}
+template <typename TC, int LDLT>
+__device__ __forceinline__ TC pivot_stored(TC p) {
+    return LDLT ? p : sqrt(p);
+}
+
+// ---------------------------------------------------------------------------
+// Elimination of the first `nel` columns of a symmetric matrix of at most
+// NR = TD * R rows by one CTA of TD x TD threads: k_small's partial
+// factorization and k_diag's block with its inverse.  Thread (tx, ty) holds
+// the entries (tx + TD i, ty + TD j), i >= j, in registers; columns go four
+// at a time:
+//   publish  the owners of columns k .. k + 3 write them to shared memory;
+//   solve    thread t < NR factors the 4 x 4 pivot block (every one the same,
+//            in registers) and solves row t's four entries against it; they go
+//            to F and, as one quad a row, to lb (LDLt: times the pivots to rq,
+//            the right factor);
+//   update   every thread subtracts the four rank-1 products from its
+//            entries, columns in order.  Entries of finished rows and columns
+//            take junk: nothing reads them again.
+// The pivots are checked, and the diagonal stored, after the last quad.
+// INV: the same steps applied to the identity give X = L^-1 (unit diagonal
+// for LDLt) in the registers of the finished columns: a second group of NR
+// threads solves X's four pivot rows beside the row group, one column each,
+// into rq and X, and the update is the same for A's and X's entries.
+// What bounds it is the chain of pivots (reciprocal square root, scale and
+// update within the quad, two barriers around it), then shared-memory reads of
+// the quads in the update (two rows a warp: 128 bytes a cycle and SM).  So
+// nothing else is on the chain, its code is straight-line, and one rolled
+// loop of a few hundred instructions serves all quads: a CTA runs it once, and
+// its instructions come from L2.  64 x 64 block with its inverse, one CTA, per
+// launch: FP64 Cholesky 36 -> 14 us, LDLt 38 -> 19 us, FP32 17.6 -> 10.7 us
+// and 23.4 -> 14.1 us (before: panels of sixteen columns factored by one
+// warp's shuffles, the inverse after them).  A small front's launch in a
+// narrow level: 44 -> 13 us (before: a right-looking loop in shared memory,
+// two divisions an entry, a barrier a column and a memory trip a child).
+// Measured slower: the matrix in shared memory instead of registers (29 us for
+// the FP64 LDLt block: aliased loads and stores wait for one another), the
+// panel one quad ahead of the update in warps of its own (26 us: the panel
+// threads then redo part of the update), a copy of the step per 16 columns
+// (23 us: instruction fetches).
+// Each entry gets the right-looking order's operations, one rounding per
+// product and update, whatever TD and R are.
+// ---------------------------------------------------------------------------
+template <typename TC>
+struct __align__(16) Quad {
+    TC v[4];
+};
+
+// shared-memory scratch of eliminate()
+template <typename TC, int NR, bool INV>
+struct __align__(16) ElimBufs {
+    Quad<TC> lb[NR + 1], rq[NR];
+    TC cb[4 * NR];
+    TC xb[INV ? 4 * NR : 1];
+    TC diag0[NR];    // |a_kk| on entry (single-precision pivot check)
+    TC piv[NR + 4];  // pivots, then stored diagonal entries
+    double sgn[NR];  // requested pivot signs (LDLt)
+    int bad;
+};
+
+template <typename TC, int LDLT, int TD, int R, bool INV, bool REG>
+__device__ __forceinline__ int eliminate(TC (&a)[R][R], int nrow, int nel, TC* F, int ldf, TC* X, int ldx,
+                                         ElimBufs<TC, TD * R, INV>& s, const Reg& reg, bool check, int* flag) {
+    constexpr int NR = TD * R;
+    static_assert(TD * TD >= (INV ? 2 : 1) * NR, "one thread per row (and per inverse column)");
+    const int tid = threadIdx.x, tx = tid % TD, ty = tid / TD;
+    if (tid == 0) s.bad = INT_MAX;
+#pragma unroll 1
+    for (int k = 0; k < nel; k += 4) {
+        const int jb = k / TD, kk = k % TD, nc = nel - k;  // columns of the quad past nc take pivot 1 and zero factors
+        {
+            const int c = ty - kk, r = tx - kk;
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+                if (j == jb) {  // uniform
+                    if (c >= 0 && c < 4)
+#pragma unroll
+                        for (int i = j; i < R; ++i) {
+                            s.cb[c * NR + tx + TD * i] = a[i][j];
+                            if (INV) a[i][j] = TC(0);
+                        }
+                    if (INV && r >= 0 && r < 4)
+#pragma unroll
+                        for (int j2 = 0; j2 <= j; ++j2) s.xb[INV ? r * NR + ty + TD * j2 : 0] = a[j][j2];
+                }
         }
         __syncthreads();
-    }
-    // right-looking partial factorization of the first nn columns, one
-    // block barrier per column: step k reads column k unscaled and scales
-    // its entries on the fly (the same rounded products the stored scaled
-    // column holds), and column k is written back scaled -- with its
-    // diagonal entry -- during step k + 1, which touches only columns > k
-    TC pk = TC(0), ik = TC(0);  // the previous column's stored diagonal and reciprocal
-    for (int k = 0; k < nn; ++k) {
-        if (k > 0) {
-            if (tid == 0) F[(k - 1) + (k - 1) * nj] = pk;
-            for (int i = k + tid; i < nj; i += nt) F[i + (k - 1) * nj] *= ik;
+        if (tid < (INV ? 2 : 1) * NR) {
+            // straight-line: a branch in here would sit on the pivot chain
+            const bool row = !INV || tid < NR;
+            const int t = row ? tid : tid - NR;
+            TC p[4][4], v[4], raw[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int r = c; r < 4; ++r) p[r][c] = s.cb[c * NR + k + r];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                v[c] = INV && !row ? s.xb[INV ? c * NR + t : 0] : s.cb[c * NR + t];
+                if (INV && !row && t >= k) v[c] = t == k + c ? TC(1) : TC(0);
+            }
+            Quad<TC> q, q2;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                TC piv = p[c][c];
+                if (REG) piv = (TC)reg_pivot(reg, LDLT ? s.sgn[min(k + c, NR - 1)] : 1.0, (double)piv);
+                if (c > 0) piv = c < nc ? piv : TC(1);
+                raw[c] = piv;
+                // after a rejected pivot the remaining steps run on junk and are discarded
+                const TC ik = pivot_recip<LDLT>(piv);
+                TC lv = (LDLT && INV && !row) ? v[c] : v[c] * ik;
+                if (c > 0) lv = c < nc ? lv : TC(0);
+#pragma unroll
+                for (int r = c + 1; r < 4; ++r) p[r][c] *= ik;
+#pragma unroll
+                for (int c2 = c + 1; c2 < 4; ++c2) {
+                    const TC l = p[c2][c];
+                    const TC lc = LDLT ? l * piv : l;
+#pragma unroll
+                    for (int r = c2; r < 4; ++r) p[r][c2] -= p[r][c] * lc;
+                    v[c2] -= lv * ((LDLT && INV && !row) ? l : lc);
+                }
+                q.v[c] = lv;
+                if (LDLT) q2.v[c] = lv * piv;
+            }
+            s.lb[INV && !row ? NR : t] = q;  // (the inverse's threads write a spare slot)
+            if (INV) {
+                // right factors: the inverse's rows in finished columns, the factor's in the rest
+                if (row == (t >= k + 4)) s.rq[t] = (LDLT && row) ? q2 : q;
+            } else if (LDLT) {
+                s.rq[t] = q2;
+            }
+            if (row) {
+                if (t > k + 3 && t < nrow) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (c < nc) F[t + (k + c) * ldf] = q.v[c];
+                } else if (t < nrow) {  // the quad's own rows
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (c < nc && t > k + c) F[t + (k + c) * ldf] = q.v[c];
+                }
+            } else if (t < k + 4) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (c < nc && t <= k + c) X[(k + c) + t * ldx] = q.v[c];
+            }
+            if (tid == 0)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s.piv[k + c] = raw[c];
         }
-        TC piv = F[k + k * nj];
-        double s = pivot_sign(signs, LDLT, f.col0 + k);
-        if (reg.delta >= 0.0) {
-            piv = (TC)reg_pivot(reg, s, (double)piv);
-            if (piv == TC(0)) return k;  // uniform across the block
-        } else if (!pivot_ok(s, (double)piv) || (!LDLT && !(piv > TC(0)))) {
-            return k;  // uniform across the block
-        }
-        if (check && tid == 0) {
-            // the original diagonal entry of column k is still in the panel
-            const double a0 = fabs((double)Pj[k + (int64_t)k * ld]);
-            const double ap = fabs((double)piv);
-            if (ap < kRescueSmall * a0 || ap > kRescueGrowth * fmax(a0, 1.0)) *flag = 1;
-        }
-        TC dk = LDLT ? piv : sqrt(piv);
-        TC inv = TC(1) / dk;
-        const int m = nj - k - 1;
-        for (int i = tid; i < m * m; i += nt) {
-            int r = k + 1 + i % m, c = k + 1 + i / m;
-            if (r >= c) {
-                TC lc = F[c + k * nj] * inv;
-                if (LDLT) lc *= piv;
-                const TC lr = F[r + k * nj] * inv;
-                F[r + c * nj] -= lr * lc;
+        __syncthreads();
+        Quad<TC> lr[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) lr[i] = s.lb[tx + TD * i];
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            if (INV || j >= jb) {  // uniform
+                const Quad<TC> u = (LDLT || INV) ? s.rq[ty + TD * j] : s.lb[ty + TD * j];
+#pragma unroll
+                for (int i = j; i < R; ++i)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) a[i][j] -= lr[i].v[c] * u.v[c];
             }
         }
-        pk = LDLT ? piv : dk;
-        ik = inv;
+    }
+    __syncthreads();
+    // the pivots: the first rejected one, and the stored diagonal
+    if (tid < nel) {
+        const TC piv = s.piv[tid];
+        const double sg = LDLT ? s.sgn[tid] : 1.0;
+        const bool bad = REG ? piv == TC(0) : !pivot_ok(sg, (double)piv) || (!LDLT && !(piv > TC(0)));
+        if (bad) atomicMin(&s.bad, tid);
+        const TC dk = pivot_stored<TC, LDLT>(piv);
+        F[tid + tid * ldf] = dk;
+        s.piv[tid] = dk;
+        if (check) {
+            const double a0 = (double)s.diag0[tid], ap = fabs((double)piv);
+            if (ap < kRescueSmall * a0 || ap > kRescueGrowth * fmax(a0, 1.0)) *flag = 1;
+        }
+    }
+    __syncthreads();
+    return s.bad == INT_MAX ? -1 : s.bad;
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
+// A small front assembled in shared memory (F, leading dimension f.ldp): the
+// panel, zeros in the update part, then the children in the reference's
+// reverse order (cholesky.jl:506-514).  The panel and every child's update
+// matrix are contiguous 16-byte-aligned blocks (leading dimensions and
+// offsets are multiples of four entries), so they stream into shared memory
+// as 16-byte asynchronous copies, as many children at a time as `stage`
+// entries hold (at least the largest one), and the adds wait for one memory
+// trip per group instead of one per child.  Ends with a block barrier.
+template <typename T>
+__device__ __forceinline__ void small_assemble(T* F, T* S, int stage, const Front& f,
+                                               const Front* __restrict__ fronts, const int32_t* __restrict__ reltgt,
+                                               const int32_t* __restrict__ chdtgt, const T* __restrict__ P,
+                                               const T* __restrict__ M) {
+    constexpr int V = 16 / (int)sizeof(T);
+    const int nn = f.nn, nj = nn + f.na, ld = f.ldp;
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    // the children's records, kSmallKids at a time, in the order they are added
+    __shared__ int kid_na[kSmallKids], kid_lm[kSmallKids], kid_sep0[kSmallKids], kid_at[kSmallKids + 1];
+    __shared__ int64_t kid_moff[kSmallKids];
+    __shared__ int32_t kid_rel[kSmallKids * kSmallMax];
+    __shared__ int kid_end;
+    const int nch = f.chd1 - f.chd0;
+    for (int i = V * tid; i < ld * nn; i += V * nt) cp_async16(F + i, P + f.poff + i);
+    for (int i = ld * nn + tid; i < ld * nj; i += nt) F[i] = T(0);
+    for (int k0 = 0; k0 < nch; k0 += kSmallKids) {
+        const int m = min(kSmallKids, nch - k0);
+        for (int q = tid; q < m; q += nt) {
+            const Front fc = fronts[chdtgt[f.chd1 - 1 - k0 - q]];
+            kid_na[q] = fc.na;
+            kid_lm[q] = fc.ldm;
+            kid_sep0[q] = fc.sep0;
+            kid_moff[q] = fc.moff;
+        }
+        __syncthreads();
+        for (int q0 = 0; q0 < m;) {
+            if (tid == 0) {  // the children of this group and where they land
+                int at = 0, q = q0;
+                while (q < m && (q == q0 || at + kid_lm[q] * kid_na[q] <= stage)) {
+                    kid_at[q] = at;
+                    at += kid_lm[q] * kid_na[q];
+                    ++q;
+                }
+                kid_end = q;
+            }
+            __syncthreads();
+            const int q1 = kid_end;
+            for (int q = q0; q < q1; ++q) {
+                const int n = kid_lm[q] * kid_na[q];
+                const T* src = M + kid_moff[q];
+                T* dst = S + kid_at[q];
+                for (int i = V * tid; i < n; i += V * nt) cp_async16(dst + i, src + i);
+                const int32_t* rel = reltgt + kid_sep0[q];
+                for (int i = tid; i < kid_na[q]; i += nt) cp_async4(kid_rel + q * kSmallMax + i, rel + i);
+            }
+            cp_async_wait_all();
+            __syncthreads();
+            for (int q = q0; q < q1; ++q) {
+                const int ma = kid_na[q], lm = kid_lm[q];
+                const int32_t* rel = kid_rel + q * kSmallMax;
+                const T* Mc = S + kid_at[q];
+                for (int b = warp; b < ma; b += nw) {
+                    T* col = F + rel[b] * ld;
+                    for (int r = b + lane; r < ma; r += 32) col[rel[r]] += Mc[r + b * lm];
+                }
+                __syncthreads();
+            }
+            q0 = q1;
+        }
+    }
+    if (nch == 0) {
+        cp_async_wait_all();
         __syncthreads();
     }
-    if (nn > 0) {
-        if (tid == 0) F[(nn - 1) + (nn - 1) * nj] = pk;
-        for (int i = nn + tid; i < nj; i += nt) F[i + (nn - 1) * nj] *= ik;
+}
+
+// The FP64 redo of a flagged single-precision small front (rare): assembled
+// and factored right-looking in shared memory as doubles (F, leading
+// dimension nj).  Returns the first rejected pivot (front-local) or -1,
+// uniform across the block.
+template <int LDLT>
+__device__ __noinline__ int small_redo(double* F, const Front& f, const Front* __restrict__ fronts,
+                                       const int32_t* __restrict__ reltgt, const int32_t* __restrict__ chdtgt,
+                                       const float* __restrict__ P, const float* __restrict__ M,
+                                       const double* __restrict__ signs) {
+    const int nn = f.nn, nj = nn + f.na;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    for (int i = tid; i < nj * nj; i += nt) {
+        const int r = i % nj, c = i / nj;
+        F[i] = c < nn ? (double)P[f.poff + r + (int64_t)c * f.ldp] : 0.0;
+    }
+    __syncthreads();
+    for (int q = f.chd1 - 1; q >= f.chd0; --q) {
+        const Front fc = fronts[chdtgt[q]];
+        const int32_t* rel = reltgt + fc.sep0;
+        for (int i = tid; i < fc.na * fc.na; i += nt) {
+            const int a = i % fc.na, b = i / fc.na;
+            if (a >= b) F[rel[a] + rel[b] * nj] += (double)M[fc.moff + a + b * fc.ldm];
+        }
+        __syncthreads();
+    }
+    for (int k = 0; k < nn; ++k) {
+        const double piv = F[k + k * nj];
+        const double s = pivot_sign(signs, LDLT, f.col0 + k);
+        if (!pivot_ok(s, piv) || (!LDLT && !(piv > 0.0))) return k;  // uniform across the block
+        const double inv = pivot_recip<LDLT>(piv);
+        __syncthreads();
+        if (tid == 0) F[k + k * nj] = pivot_stored<double, LDLT>(piv);
+        for (int i = k + 1 + tid; i < nj; i += nt) F[i + k * nj] *= inv;
+        __syncthreads();
+        const int m = nj - k - 1;
+        for (int i = tid; i < m * m; i += nt) {
+            const int r = k + 1 + i % m, c = k + 1 + i / m;
+            if (r >= c) {
+                double lc = F[c + k * nj];
+                if (LDLT) lc *= piv;
+                F[r + c * nj] -= F[r + k * nj] * lc;
+            }
+        }
         __syncthreads();
     }
     return -1;
 }
 
-// Write a factored small front back: panel, update matrix, LDLt pivots (the
-// diagonal of the factored panel holds them: the unit diagonal of L is
-// implied and the LDLt panel diagonal keeps d_k).
+// Write a factored small front's panel (F, leading dimension lf) and LDLt
+// pivots back (the panel diagonal holds them: the unit diagonal of L is
+// implied).
 template <typename TC, typename T, int LDLT>
-__device__ void small_front_store(const TC* F, const Front& f, T* __restrict__ P, T* __restrict__ M,
-                                 T* __restrict__ d) {
-    const int nn = f.nn, na = f.na, nj = nn + na, ld = f.ldp;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    T* Pj = P + f.poff;
-    for (int i = tid; i < nj * nn; i += nt) {
-        int r = i % nj, c = i / nj;
-        Pj[r + (int64_t)c * ld] = (T)F[i];
+__device__ __forceinline__ void small_panel_store(const TC* F, int lf, const Front& f, T* __restrict__ P,
+                                                  T* __restrict__ d) {
+    const int nn = f.nn, nj = nn + f.na;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int c = warp; c < nn; c += nw) {
+        T* dst = P + f.poff + (int64_t)c * f.ldp;
+        for (int r = c + lane; r < nj; r += 32) dst[r] = (T)F[r + c * lf];
     }
     if (LDLT)
-        for (int k = tid; k < nn; k += nt) d[f.col0 + k] = (T)F[k + k * nj];
-    T* Mj = M + f.moff;
-    const int lm = f.ldm;
-    for (int i = tid; i < na * na; i += nt) {
-        int a = i % na, b = i / na;
-        Mj[a + b * lm] = (T)F[(nn + a) + (nn + b) * nj];
-    }
+        for (int k = threadIdx.x; k < nn; k += blockDim.x) d[f.col0 + k] = (T)F[k + k * lf];
 }
 
-// small fronts (nj <= kSmallMax): one CTA holds the whole front in shared
-// memory.  Single precision: a front whose factorization rejects a pivot or
-// flags a small or grown pivot is factored again from its inputs in FP64 in
-// the same shared memory (fronts of nj <= kSmallRescue, whose FP64 front fits
-// the FP32 buffer; the panel and the children's update matrices are only
-// read before the final store, so the inputs are intact), and the FP64
+// small fronts (nj <= kSmallMax): one CTA of TD x TD threads assembles the
+// front in shared memory and eliminates it in registers (eliminate()).  Single precision: a
+// front whose factorization rejects a pivot or flags a small or grown pivot
+// is factored again from its inputs in FP64 in the same shared memory (fronts
+// of nj <= kSmallRescue; the panel and the children's update matrices are
+// only read before the final store, so the inputs are intact), and the FP64
 // result is stored rounded to FP32.  A rejection in FP64 -- or in FP32 for a
 // larger front -- is reported through info.
-constexpr int kSmallRescue = 67;  // 67^2 doubles <= kSmallMax^2 floats
-constexpr int kSmallNarrowNJ = 48;     // levels whose small fronts all have nj <= this ...
-constexpr int kSmallWideLevel = 4 * 148;  // ... and that hold at least this many run 128-thread CTAs,
-constexpr int kSmallTinyNJ = 32;       // 64-thread CTAs when nj <= this
+constexpr int kSmallRescue = 67;
 
-template <typename T, int LDLT>
-__global__ void __launch_bounds__(256) k_small(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                               const int32_t* __restrict__ reltgt,
-                                               const int32_t* __restrict__ chdtgt, T* __restrict__ P,
-                                               T* __restrict__ M, T* __restrict__ d,
-                                               const double* __restrict__ signs, long long* __restrict__ info,
-                                               int* __restrict__ rescued, Reg reg) {
+template <typename T, int LDLT, int TD, int R, bool REG>
+__global__ void __launch_bounds__(TD * TD) k_small(const Front* __restrict__ fronts, const Item* __restrict__ items,
+                                                   int stage, const int32_t* __restrict__ reltgt,
+                                                   const int32_t* __restrict__ chdtgt, T* __restrict__ P,
+                                                   T* __restrict__ M, T* __restrict__ d,
+                                                   const double* __restrict__ signs, long long* __restrict__ info,
+                                                   int* __restrict__ rescued, Reg reg) {
     pdl_prologue();
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ ElimBufs<T, TD * R, false> s;
     __shared__ int flag;
-    T* F = reinterpret_cast<T*>(smem_raw);
+    T* S = reinterpret_cast<T*>(smem_raw);  // staged children
+    T* F = S + stage;
     const Item it = items[blockIdx.x];
     const Front f = fronts[it.front];
-    const int nj = f.nn + f.na;
+    const int nn = f.nn, na = f.na, nj = nn + na;
+    const int tid = threadIdx.x, tx = tid % TD, ty = tid / TD;
     constexpr bool single = sizeof(T) == 4;
-    if (threadIdx.x == 0) flag = 0;
-    __syncthreads();
-    int bad = small_front<T, T, LDLT>(F, f, fronts, reltgt, chdtgt, P, M, signs, single, &flag, reg);
-    __syncthreads();
-    if (single && (bad >= 0 || flag) && nj <= kSmallRescue) {
-        double* F64 = reinterpret_cast<double*>(smem_raw);
-        bad = small_front<double, T, LDLT>(F64, f, fronts, reltgt, chdtgt, P, M, signs, false, &flag, reg);
-        if (bad < 0) {
-            if (threadIdx.x == 0) atomicAdd(rescued, 1);
-            small_front_store<double, T, LDLT>(F64, f, P, M, d);
-            return;
+    if (tid == 0) flag = 0;
+    for (int k = tid; k < nn; k += TD * TD) {
+        if (LDLT) s.sgn[k] = pivot_sign(signs, LDLT, f.col0 + k);
+        // the pivot check compares against the entry before the children's updates
+        if (single) s.diag0[k] = (T)fabs((double)P[f.poff + k + (int64_t)k * f.ldp]);
+    }
+    small_assemble<T>(F, S, stage, f, fronts, reltgt, chdtgt, P, M);
+    T a[R][R];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+            const int r = tx + TD * i, c = ty + TD * j;
+            a[i][j] = (r < nj && c <= r) ? F[r + c * f.ldp] : T(0);
+        }
+    int bad = eliminate<T, LDLT, TD, R, false, REG>(a, nj, nn, F, f.ldp, nullptr, 0, s, reg, single, &flag);
+    if constexpr (single) {
+        if ((bad >= 0 || flag) && nj <= kSmallRescue) {
+            double* F64 = reinterpret_cast<double*>(smem_raw);
+            __syncthreads();
+            bad = small_redo<LDLT>(F64, f, fronts, reltgt, chdtgt, P, M, signs);
+            if (bad < 0) {
+                if (tid == 0) atomicAdd(rescued, 1);
+                small_panel_store<double, T, LDLT>(F64, nj, f, P, d);
+                for (int i = tid; i < na * na; i += TD * TD) {
+                    const int r = i % na, c = i / na;
+                    if (r >= c) M[f.moff + r + c * f.ldm] = (T)F64[(nn + r) + (nn + c) * nj];
+                }
+                return;
+            }
         }
     }
     if (bad >= 0) {
-        if (threadIdx.x == 0) atomicMin(info, (long long)(f.col0 + bad + 1));
+        if (tid == 0) atomicMin(info, (long long)(f.col0 + bad + 1));
         return;
     }
-    small_front_store<T, T, LDLT>(F, f, P, M, d);
+    small_panel_store<T, T, LDLT>(F, f.ldp, f, P, d);
+    T* Mj = M + f.moff - nn - (int64_t)nn * f.ldm;
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+            const int r = tx + TD * i, c = ty + TD * j;
+            if (r < nj && c <= r && c >= nn) Mj[r + (int64_t)c * f.ldm] = a[i][j];
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -399,10 +665,9 @@ __device__ int warp_front(TC* F, const Front& f, const Front* __restrict__ front
             const double ap = fabs((double)piv);
             if (ap < kRescueSmall * a0 || ap > kRescueGrowth * fmax(a0, 1.0)) *flag = true;
         }
-        const TC dk = LDLT ? piv : sqrt(piv);
-        const TC inv = TC(1) / dk;
+        const TC inv = pivot_recip<LDLT>(piv);
         __syncwarp();
-        if (lane == k) F[k + k * (ROWS + 1)] = LDLT ? piv : dk;
+        if (lane == k) F[k + k * (ROWS + 1)] = pivot_stored<TC, LDLT>(piv);
         if (lane > k && row) F[lane + k * (ROWS + 1)] *= inv;
         __syncwarp();
         if (lane > k && row) {
@@ -554,443 +819,32 @@ __global__ void __launch_bounds__(256) k_ea(const Front* __restrict__ fronts, co
 // diagonal block: factor + inverse
 // ---------------------------------------------------------------------------
 
-// Diagonal block: factor + inverse, one CTA of 256 threads per front.
-//
-// The 64 x 64 block (columns >= w padded with the identity) sits in shared
-// memory and is factored in four 16-column panels.  Per panel, warp 0
-// factors the 16 x 16 diagonal block in registers (lane i < 16 owns row i;
-// column k reaches the other lanes by shuffles, so the 16 dependent pivot
-// steps use no barrier) and inverts it (lane j owns column j).  All threads
-// then form the rows below as A L^-T (D^-1) with that inverse and apply the
-// rank-16 update to the trailing block; both are fully unrolled 16-term dot
-// products.  Finally the off-diagonal 16 x 16 blocks of X = L^-1 (unit
-// diagonal for LDLt) follow along the block sub-diagonals,
-// X_ij = -X_ii sum_{k=j}^{i-1} L_ik X_kj.  About 26 barriers in all.  This is
-// diag_block_seq (the FP64 kernel); the FP32 kernel runs diag_block_la,
-// which takes the inverses and the bulk updates off warp 0's chain.
+// Diagonal block: factor + inverse, one CTA of 256 threads per front
+// (eliminate() on the 64 x 64 block, columns >= w padded with the identity).
 constexpr int LDS = kNB + 4;  // shared-memory leading dimension of the GEMM stages
-constexpr int LDA = kNB + 1;  // leading dimension of the block and its inverse in the diagonal kernel
+constexpr int LDA = kNB + 1;  // leading dimension of the factor and inverse in the diagonal kernel
+constexpr int kDiagTD = 16, kDiagR = kNB / kDiagTD;
 
 // dynamic shared memory of k_diag: the FP64 layout in both precisions (the
 // single-precision kernel refactors flagged blocks in FP64 in place)
 template <typename T>
-constexpr int diag_smem() { return (2 * kNB * LDA + 2 * kNB) * (int)sizeof(double); }
-
-// The pivot's diagonal entry dk (sqrt(p) for Cholesky, p for LDLt) and its
-// reciprocal.  FP32 (the mixed form, whose factor only preconditions the
-// FP64 refinement) uses the hardware reciprocal square root / reciprocal;
-// FP64 keeps the correctly rounded operations of the plain form.
-template <typename T, int LDLT>
-__device__ __forceinline__ void diag_pivot(T p, T& dk, T& ik);
-template <>
-__device__ __forceinline__ void diag_pivot<float, 0>(float p, float& dk, float& ik) {
-    ik = rsqrtf(p);
-    dk = p * ik;
-}
-template <>
-__device__ __forceinline__ void diag_pivot<float, 1>(float p, float& dk, float& ik) {
-    dk = p;
-    ik = __frcp_rn(p);
-}
-template <>
-__device__ __forceinline__ void diag_pivot<double, 0>(double p, double& dk, double& ik) {
-    dk = sqrt(p);
-    ik = 1.0 / dk;
-}
-template <>
-__device__ __forceinline__ void diag_pivot<double, 1>(double p, double& dk, double& ik) {
-    dk = p;
-    ik = 1.0 / p;
-}
+constexpr int diag_smem() { return 2 * kNB * LDA * (int)sizeof(double) + (int)sizeof(ElimBufs<double, kNB, true>); }
 
 // Factor and invert the 64 x 64 block held in shared memory as TC: A (block,
-// identity beyond column w), X (inverse), pivs (L_kk or d_k), rinv (their
-// reciprocals).  Returns the first rejected pivot (block-local) or -1,
-// uniform across the block; bad_s is a shared scratch int.
-//
-// Four 16-column panels with look-ahead.  Panel p: warp 0 factors its 16 x 16
-// diagonal block in registers (the pivot chain, by shuffles) while warps 1..7
-// apply panel p-1's update to every entry below that block (the rows and
-// columns the later panels read); then every thread with a row below solves
-// that row against the panel's triangle (forward substitution in registers),
-// and the next panel's 16 x 16 diagonal block takes panel p's update, so warp
-// 0 can start on it at once.  The chain therefore waits for no bulk update.
-// The 16 x 16 inverses (warps 0..3 at once) and the off-diagonal blocks of X
-// follow the factorization.
-template <typename TC, int LDLT>
-__device__ __forceinline__ void diag_factor16(TC* A, TC* pivs, TC* rinv, int pb, int w,
-                                              const double* __restrict__ signs, int64_t colbase, int* bad_s,
-                                              const Reg& reg, int lane) {
-    using T = TC;
-    const int i = lane & 15;  // lanes 16..31 mirror 0..15
-    T a[16];
+// identity beyond column w) and X (zeros, receives the inverse); s.piv gets
+// the stored diagonal.  Returns the first rejected pivot (block-local) or -1,
+// uniform across the block.
+template <typename TC, int LDLT, bool REG>
+__device__ __forceinline__ int diag_block(TC* A, TC* X, ElimBufs<TC, kNB, true>& s, int w,
+                                          const double* __restrict__ signs, int64_t colbase, const Reg& reg) {
+    const int tid = threadIdx.x, tx = tid % kDiagTD, ty = tid / kDiagTD;
+    if (LDLT && tid < w) s.sgn[tid] = pivot_sign(signs, LDLT, colbase + tid);
+    TC a[kDiagR][kDiagR];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) a[j] = j <= i ? A[(pb + i) + (pb + j) * LDA] : T(0);
-    T mypiv = T(1), myrinv = T(1);
-    int bad = -1;
+    for (int i = 0; i < kDiagR; ++i)
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        T pv = __shfl_sync(0xffffffffu, a[k], k);
-        if (reg.delta >= 0.0) {
-            if (pb + k < w) {
-                pv = (T)reg_pivot(reg, pivot_sign(signs, LDLT, colbase + pb + k), (double)pv);
-                if (i == k) a[k] = pv;
-                if (bad < 0 && pv == T(0)) bad = pb + k;
-            }
-        } else if (bad < 0 && pb + k < w) {
-            const double sg = pivot_sign(signs, LDLT, colbase + pb + k);
-            if (!pivot_ok(sg, (double)pv) || (!LDLT && !(pv > T(0)))) bad = pb + k;
-        }
-        // after a rejected pivot the remaining steps run on junk and are discarded
-        T dk, ik;
-        diag_pivot<T, LDLT>(pv, dk, ik);
-        const T aik = a[k];
-        const T lik = aik * ik;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            if (j > k) {  // resolved at compile time once both loops are unrolled
-                const T u = __shfl_sync(0xffffffffu, LDLT ? aik : lik, j);
-                if (i >= j) a[j] -= lik * u;
-            }
-        }
-        if (i > k) a[k] = lik;
-        else if (i == k) {
-            if (!LDLT) a[k] = dk;
-            mypiv = dk;
-            myrinv = ik;
-        }
-    }
-    if (lane < 16) {
-#pragma unroll
-        for (int jj = 0; jj < 16; ++jj)
-            if (jj <= i) A[(pb + i) + (pb + jj) * LDA] = a[jj];
-        pivs[pb + i] = mypiv;
-        rinv[pb + i] = myrinv;
-    }
-    if (lane == 0 && bad >= 0) (*bad_s) = bad;
-}
-
-// the inverse of the factored 16 x 16 diagonal block at pb (one warp): lane
-// j owns column j
-template <typename TC, int LDLT>
-__device__ __forceinline__ void diag_inv16(const TC* A, TC* X, const TC* rinv, int pb, int lane) {
-    using T = TC;
-    const int i = lane & 15, j = i;
-    T a[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) a[k] = k < i ? A[(pb + i) + (pb + k) * LDA] : T(0);
-    const T myrinv = rinv[pb + i];
-    T x[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        T acc = T(0);
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            if (k < r) {  // resolved at compile time once both loops are unrolled
-                const T lrk = __shfl_sync(0xffffffffu, a[k], r);
-                if (k >= j) acc += lrk * x[k];
-            }
-        }
-        const T rr = __shfl_sync(0xffffffffu, myrinv, r);
-        x[r] = r < j ? T(0) : (r == j ? (LDLT ? T(1) : rr) : (LDLT ? -acc : -acc * rr));
-    }
-    if (lane < 16)
-#pragma unroll
-        for (int r = 0; r < 16; ++r) X[(pb + r) + (pb + j) * LDA] = x[r];
-}
-
-// A[i, j] -= sum_q L[i, pb + q] (d_q) L[j, pb + q] over a rectangle of rows
-// [r0, 64) x columns [c0, c1), lower triangle only, threads t0.. of the block
-template <typename TC, int LDLT>
-__device__ __forceinline__ void diag_update(TC* A, const TC* pivs, int pb, int r0, int c0, int c1, int t,
-                                            int nt) {
-    using T = TC;
-    const int nr = kNB - r0, nc = c1 - c0;
-    for (int e = t; e < nr * nc; e += nt) {
-        const int i = r0 + e % nr, j = c0 + e / nr;
-        if (i >= j) {
-            T acc = T(0);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                T lj = A[j + (pb + q) * LDA];
-                if (LDLT) lj *= pivs[pb + q];
-                acc += A[i + (pb + q) * LDA] * lj;
-            }
-            A[i + j * LDA] -= acc;
-        }
-    }
-}
-
-// The off-diagonal 16 x 16 blocks of X = L^-1 from the four diagonal
-// inverses already in X, by block distance (the whole CTA).
-template <typename TC>
-__device__ __forceinline__ void diag_inv_offdiag(const TC* A, TC* X) {
-    const int tid = threadIdx.x;
-    using T = TC;
-#pragma unroll 1
-    for (int dist = 1; dist < 4; ++dist) {
-        const int nb = 4 - dist;
-        T tmp[3];
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {  // T_ij = sum_{k=j}^{i-1} L_ik X_kj
-            const int o = tid + 256 * s;
-            tmp[s] = T(0);
-            if (o < nb * 256) {
-                const int bj = o >> 8, bi = bj + dist, r = (o >> 4) & 15, c = o & 15;
-                T acc = T(0);
-                for (int bk = bj; bk < bi; ++bk)
-#pragma unroll
-                    for (int q = 0; q < 16; ++q)
-                        acc += A[(16 * bi + r) + (16 * bk + q) * LDA] * X[(16 * bk + q) + (16 * bj + c) * LDA];
-                tmp[s] = acc;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int o = tid + 256 * s;
-            if (o < nb * 256) {
-                const int bj = o >> 8, bi = bj + dist, r = (o >> 4) & 15, c = o & 15;
-                X[(16 * bi + r) + (16 * bj + c) * LDA] = tmp[s];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {  // X_ij = -X_ii T_ij
-            const int o = tid + 256 * s;
-            if (o < nb * 256) {
-                const int bj = o >> 8, bi = bj + dist, r = (o >> 4) & 15, c = o & 15;
-                T acc = T(0);
-#pragma unroll
-                for (int q = 0; q < 16; ++q)
-                    acc += X[(16 * bi + r) + (16 * bi + q) * LDA] * X[(16 * bi + q) + (16 * bj + c) * LDA];
-                tmp[s] = -acc;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int o = tid + 256 * s;
-            if (o < nb * 256) {
-                const int bj = o >> 8, bi = bj + dist, r = (o >> 4) & 15, c = o & 15;
-                X[(16 * bi + r) + (16 * bj + c) * LDA] = tmp[s];
-            }
-        }
-        __syncthreads();
-    }
-}
-
-template <typename TC, int LDLT>
-__device__ int diag_block_la(TC* A, TC* X, TC* pivs, TC* rinv, int w, const double* __restrict__ signs,
-                          int64_t colbase, int* bad_s, Reg reg) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    using T = TC;
-    if (tid == 0) *bad_s = -1;
-    __syncthreads();
-    // the panel loop stays rolled: its body runs once per panel and block,
-    // and four unrolled copies made the kernel wait on instruction fetches
-#pragma unroll 1
-    for (int p = 0; p < 4; ++p) {
-        const int pb = p * 16;
-        if (warp == 0) {
-            diag_factor16<TC, LDLT>(A, pivs, rinv, pb, w, signs, colbase, bad_s, reg, lane);
-        } else if (p > 0) {
-            // panel p-1's update of everything below the diagonal block p
-            // (rows >= pb + 16, columns pb .. row); the block itself took it
-            // at the end of the previous panel
-            diag_update<TC, LDLT>(A, pivs, pb - 16, pb + 16, pb, kNB, tid - 32, 224);
-        }
-        __syncthreads();
-        if ((*bad_s) >= 0) break;  // uniform
-        if (p == 3) break;
-        // rows below: solve each row against the panel's triangle, in four
-        // column groups (finish a group, then subtract it from the later
-        // columns at once), which cuts the dependent chain of the
-        // substitution to about a third
-        const int r = pb + 16 + tid;
-        if (r < kNB) {
-            T y[16];
-#pragma unroll
-            for (int c = 0; c < 16; ++c) y[c] = A[r + (pb + c) * LDA];
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-#pragma unroll
-                for (int c = 4 * g; c < 4 * g + 4; ++c) {
-#pragma unroll
-                    for (int q = 4 * g; q < c; ++q) y[c] -= y[q] * A[(pb + c) + (pb + q) * LDA];
-                    if (!LDLT) y[c] *= rinv[pb + c];
-                }
-#pragma unroll
-                for (int c = 4 * g + 4; c < 16; ++c)
-#pragma unroll
-                    for (int q = 4 * g; q < 4 * g + 4; ++q) y[c] -= y[q] * A[(pb + c) + (pb + q) * LDA];
-            }
-#pragma unroll
-            for (int c = 0; c < 16; ++c) A[r + (pb + c) * LDA] = LDLT ? y[c] * rinv[pb + c] : y[c];
-        }
-        __syncthreads();
-        // the next diagonal block takes this panel's update now
-        {
-            const int e = tid;
-            if (e < 256) {
-                const int ii = e & 15, jj = e >> 4;
-                const int gi = pb + 16 + ii, gj = pb + 16 + jj;
-                if (ii >= jj) {
-                    T acc = T(0);
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        T lj = A[gj + (pb + q) * LDA];
-                        if (LDLT) lj *= pivs[pb + q];
-                        acc += A[gi + (pb + q) * LDA] * lj;
-                    }
-                    A[gi + gj * LDA] -= acc;
-                }
-            }
-        }
-        __syncthreads();
-    }
-    if (*bad_s >= 0) return *bad_s;  // uniform
-    // the four 16 x 16 diagonal inverses at once
-    if (warp < 4) diag_inv16<TC, LDLT>(A, X, rinv, warp * 16, lane);
-    __syncthreads();
-    diag_inv_offdiag<TC>(A, X);
-    return -1;
-}
-
-// The sequential version: per panel, warp 0 factors and inverts the 16 x 16
-// diagonal block, then the CTA forms the rows below from that inverse and
-// applies the panel's trailing update.
-template <typename TC, int LDLT>
-__device__ int diag_block_seq(TC* A, TC* X, TC* pivs, TC* rinv, int w, const double* __restrict__ signs,
-                          int64_t colbase, int* bad_s, Reg reg) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    using T = TC;
-    if (tid == 0) *bad_s = -1;
-    __syncthreads();
-#pragma unroll 1
-    for (int p = 0; p < 4; ++p) {
-        const int pb = p * 16;
-        if (warp == 0) {
-            const int i = lane & 15;  // lanes 16..31 mirror 0..15
-            T a[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) a[j] = j <= i ? A[(pb + i) + (pb + j) * LDA] : T(0);
-            T mypiv = T(1), myrinv = T(1);
-            int bad = -1;
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                T pv = __shfl_sync(0xffffffffu, a[k], k);
-                if (reg.delta >= 0.0) {
-                    if (pb + k < w) {
-                        pv = (T)reg_pivot(reg, pivot_sign(signs, LDLT, colbase + pb + k), (double)pv);
-                        if (i == k) a[k] = pv;
-                        if (bad < 0 && pv == T(0)) bad = pb + k;
-                    }
-                } else if (bad < 0 && pb + k < w) {
-                    const double sg = pivot_sign(signs, LDLT, colbase + pb + k);
-                    if (!pivot_ok(sg, (double)pv) || (!LDLT && !(pv > T(0)))) bad = pb + k;
-                }
-                // after a rejected pivot the remaining steps run on junk and are discarded
-                T dk, ik;
-                diag_pivot<T, LDLT>(pv, dk, ik);
-                const T aik = a[k];
-                const T lik = aik * ik;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    if (j > k) {  // resolved at compile time once both loops are unrolled
-                        const T u = __shfl_sync(0xffffffffu, LDLT ? aik : lik, j);
-                        if (i >= j) a[j] -= lik * u;
-                    }
-                }
-                if (i > k) a[k] = lik;
-                else if (i == k) {
-                    if (!LDLT) a[k] = dk;
-                    mypiv = dk;
-                    myrinv = ik;
-                }
-            }
-            // inverse of the 16 x 16 factor: lane j owns column j
-            const int j = i;
-            T x[16];
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                T acc = T(0);
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    if (k < r) {  // resolved at compile time once both loops are unrolled
-                        const T lrk = __shfl_sync(0xffffffffu, a[k], r);
-                        if (k >= j) acc += lrk * x[k];
-                    }
-                }
-                const T rr = __shfl_sync(0xffffffffu, myrinv, r);
-                x[r] = r < j ? T(0) : (r == j ? (LDLT ? T(1) : rr) : (LDLT ? -acc : -acc * rr));
-            }
-            if (lane < 16) {
-#pragma unroll
-                for (int jj = 0; jj < 16; ++jj)
-                    if (jj <= i) A[(pb + i) + (pb + jj) * LDA] = a[jj];
-#pragma unroll
-                for (int r = 0; r < 16; ++r) X[(pb + r) + (pb + j) * LDA] = x[r];
-                pivs[pb + i] = mypiv;
-                rinv[pb + i] = myrinv;
-            }
-            if (lane == 0 && bad >= 0) (*bad_s) = bad;
-        }
-        __syncthreads();
-        if ((*bad_s) >= 0) break;  // uniform
-        const int m = 48 - pb;  // rows / columns after the panel
-        if (m == 0) break;
-        // rows below: L_rc = sum_{q <= c} A_r,pb+q Xpp_c,q (/ d_c)
-        T res[3];
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int o = tid + 256 * s;
-            res[s] = T(0);
-            if (o < m * 16) {
-                const int r = pb + 16 + o % m, c = o / m;
-                T acc = T(0);
-#pragma unroll
-                for (int q = 0; q < 16; ++q) acc += A[r + (pb + q) * LDA] * X[(pb + c) + (pb + q) * LDA];
-                res[s] = LDLT ? acc * rinv[pb + c] : acc;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int o = tid + 256 * s;
-            if (o < m * 16) A[(pb + 16 + o % m) + (pb + o / m) * LDA] = res[s];
-        }
-        __syncthreads();
-        // trailing update A_ij -= sum_q L_iq (d_q) L_jq, pb+16 <= j <= i
-        for (int e = tid; e < m * m; e += 256) {
-            const int i = pb + 16 + e % m, j = pb + 16 + e / m;
-            if (i >= j) {
-                T acc = T(0);
-#pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    T lj = A[j + (pb + q) * LDA];
-                    if (LDLT) lj *= pivs[pb + q];
-                    acc += A[i + (pb + q) * LDA] * lj;
-                }
-                A[i + j * LDA] -= acc;
-            }
-        }
-        __syncthreads();
-    }
-    if (*bad_s >= 0) return *bad_s;  // uniform
-    diag_inv_offdiag<TC>(A, X);
-    return -1;
-}
-
-// FP32 (the mixed form) takes the look-ahead version; FP64 the sequential
-// one, measured faster for doubles (the look-ahead's update warps compete
-// with warp 0's pivot chain for the FP64 pipes, and the row substitution is
-// a longer FP64 dependency chain than the product with the inverse).
-template <typename TC, int LDLT>
-__device__ int diag_block(TC* A, TC* X, TC* pivs, TC* rinv, int w, const double* __restrict__ signs,
-                          int64_t colbase, int* bad_s, Reg reg) {
-    if (sizeof(TC) == 4) return diag_block_la<TC, LDLT>(A, X, pivs, rinv, w, signs, colbase, bad_s, reg);
-    return diag_block_seq<TC, LDLT>(A, X, pivs, rinv, w, signs, colbase, bad_s, reg);
+        for (int j = 0; j <= i; ++j) a[i][j] = A[(tx + kDiagTD * i) + (ty + kDiagTD * j) * LDA];
+    return eliminate<TC, LDLT, kDiagTD, kDiagR, true, REG>(a, kNB, w, A, LDA, X, LDA, s, reg, false, nullptr);
 }
 
 // Write back a factored diagonal block: the factor into the panel, the LDLt
@@ -1013,7 +867,7 @@ __device__ void diag_block_store(const TC* A, const TC* X, const TC* pivs, int w
 }
 
 template <typename TC, typename T>
-__device__ void diag_block_load(TC* A, TC* X, const T* Pj, int64_t ld, int c0, int w) {
+__device__ __forceinline__ void diag_block_load(TC* A, TC* X, const T* Pj, int64_t ld, int c0, int w) {
     const int tid = threadIdx.x;
 #pragma unroll
     for (int e = tid; e < kNB * kNB; e += 256) {
@@ -1031,18 +885,19 @@ __device__ void diag_block_load(TC* A, TC* X, const T* Pj, int64_t ld, int c0, i
 // the block is loaded again and factored and inverted in FP64 (the dynamic
 // shared memory is sized for that), and the FP64 result is stored rounded to
 // FP32.  A rejection in FP64 is reported through info.
-template <typename T, int LDLT>
+template <typename T, int LDLT, bool REG>
 __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ fronts, const Item* __restrict__ items,
                                               int c0, T* __restrict__ P, T* __restrict__ inv,
                                               T* __restrict__ d, const double* __restrict__ signs,
                                               long long* __restrict__ info, int* __restrict__ rescued, Reg reg) {
     pdl_prologue();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* A = reinterpret_cast<T*>(smem_raw);  // block, A[r + c * LDA]
+    T* A = reinterpret_cast<T*>(smem_raw);  // block, then its factor, A[r + c * LDA]
     T* X = A + kNB * LDA;                   // inverse, same layout
-    T* pivs = X + kNB * LDA;                // L_kk (Cholesky) or d_k (LDLt)
-    T* rinv = pivs + kNB;                   // 1 / L_kk or 1 / d_k
-    __shared__ int bad_s, flag_s;
+    unsigned char* sraw = smem_raw + 2 * kNB * LDA * sizeof(double);
+    ElimBufs<T, kNB, true>& s = *reinterpret_cast<ElimBufs<T, kNB, true>*>(sraw);
+    const T* pivs = s.piv;  // L_kk (Cholesky) or d_k (LDLt)
+    __shared__ int flag_s;
     __shared__ double dmax_s;
     const Item it = items[blockIdx.x];
     const Front f = fronts[it.front];
@@ -1057,11 +912,11 @@ __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ front
     diag_block_load<T, T>(A, X, Pj, ld, c0, w);
     __syncthreads();
     // |a_kk| before the factorization and the block's largest (non-negative
-    // doubles order like their bit patterns); diag_block starts with a barrier
+    // doubles order like their bit patterns); the factorization has barriers
     const double a0 = tid < w ? fabs((double)A[tid + tid * LDA]) : 0.0;
     if (single && tid < w)
         atomicMax(reinterpret_cast<unsigned long long*>(&dmax_s), (unsigned long long)__double_as_longlong(a0));
-    int bad = diag_block<T, LDLT>(A, X, pivs, rinv, w, signs, (int64_t)f.col0 + c0, &bad_s, reg);
+    int bad = diag_block<T, LDLT, REG>(A, X, s, w, signs, (int64_t)f.col0 + c0, reg);
     if (single) {
         if (bad < 0 && tid < w) {
             const double dk = LDLT ? fabs((double)pivs[tid]) : (double)pivs[tid] * (double)pivs[tid];
@@ -1071,14 +926,14 @@ __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ front
         if (bad >= 0 || flag_s) {
             double* A64 = reinterpret_cast<double*>(smem_raw);
             double* X64 = A64 + kNB * LDA;
-            double* piv64 = X64 + kNB * LDA;
-            double* rinv64 = piv64 + kNB;
+            ElimBufs<double, kNB, true>& s64 = *reinterpret_cast<ElimBufs<double, kNB, true>*>(sraw);
             __syncthreads();
             diag_block_load<double, T>(A64, X64, Pj, ld, c0, w);
-            bad = diag_block<double, LDLT>(A64, X64, piv64, rinv64, w, signs, (int64_t)f.col0 + c0, &bad_s, reg);
+            __syncthreads();
+            bad = diag_block<double, LDLT, false>(A64, X64, s64, w, signs, (int64_t)f.col0 + c0, reg);
             if (bad < 0) {
                 if (tid == 0) atomicAdd(rescued, 1);
-                diag_block_store<double, T, LDLT>(A64, X64, piv64, w, Pj, ld, c0, d, f.col0 + c0, dst);
+                diag_block_store<double, T, LDLT>(A64, X64, s64.piv, w, Pj, ld, c0, d, f.col0 + c0, dst);
                 return;
             }
         }
@@ -1513,19 +1368,43 @@ int launch_panel32_to_dl(mf_handle* h, double* dD, double* dL) {
 }
 
 
-template <typename T, int LDLT>
+// k_small over one run of a level's small fronts of at most mj rows: 64
+// threads up to 48 rows (two warps keep the barriers of the pivot chain
+// short), 256 above.  Shared memory holds `stage` staged
+// entries of children and a front of mj rows (as FP64 up to kSmallRescue
+// rows, for the in-place rescue of an FP32 front).
+template <typename T, int LDLT, bool REG, int TD, int R>
+static int small_go(mf_handle* h, const ItemList& l, int mj, int stage, const FactorBufs<T>& fb, const Reg& reg) {
+    const int rj = std::min(mj, kSmallRescue), lj = (mj + 3) & ~3;
+    const size_t sm = std::max<size_t>(((size_t)stage + (size_t)lj * mj) * sizeof(T), sizeof(T) == 4 ? (size_t)rj * rj * 8 : 0);
+    MF_CUDA(cudaFuncSetAttribute(k_small<T, LDLT, TD, R, REG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (kSmallStage + kSmallMax * kSmallMax) * (int)sizeof(T)));
+    launch_k(k_small<T, LDLT, TD, R, REG>, grid_for(l.cnt), TD * TD, sm, h->stream, h->d_fronts,
+             h->d_items + l.off, stage, h->d_reltgt, h->d_chdtgt, fb.P, fb.M, fb.d, h->d_signs, h->d_info,
+             h->d_rescued, reg);
+    MF_CUDA(cudaGetLastError());
+    return 0;
+}
+
+template <typename T, int LDLT, bool REG>
+static int launch_small(mf_handle* h, const ItemList& l, int mj, int stage, const FactorBufs<T>& fb, const Reg& reg) {
+    if (mj <= 32) return small_go<T, LDLT, REG, 8, 4>(h, l, mj, stage, fb, reg);
+    if (mj <= 48) return small_go<T, LDLT, REG, 8, 6>(h, l, mj, stage, fb, reg);
+    if (mj <= 64) return small_go<T, LDLT, REG, 16, 4>(h, l, mj, stage, fb, reg);
+    return small_go<T, LDLT, REG, 16, 6>(h, l, mj, stage, fb, reg);
+}
+
+template <typename T, int LDLT, bool REG>
 static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
     // the pivot rule applies to the FP64 factorization; the mixed form keeps
     // NoRegularization (its single-precision factor only preconditions)
     const Reg reg = std::is_same<T, double>::value ? h->reg : Reg();
     constexpr int gs = gemm_smem<T>();
-    MF_CUDA(cudaFuncSetAttribute(k_small<T, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmallMax * kSmallMax * (int)sizeof(T)));
     MF_CUDA(cudaFuncSetAttribute(k_small_warp<T, LDLT, kWarpSmallNJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kWarpFronts * warp_slice<kWarpSmallNJ>()));
     MF_CUDA(cudaFuncSetAttribute(k_small_warp<T, LDLT, kWarpSmallNJ2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kWarpFronts * warp_slice<kWarpSmallNJ2>()));
-    MF_CUDA(cudaFuncSetAttribute(k_diag<T, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<T>()));
+    MF_CUDA(cudaFuncSetAttribute(k_diag<T, LDLT, REG>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<T>()));
     MF_CUDA(cudaFuncSetAttribute(k_inv256<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, inv256_smem<T>()));
     MF_CUDA(cudaFuncSetAttribute(k_gemm<T, G_LEFT, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs));
     MF_CUDA(cudaFuncSetAttribute(k_gemm<T, G_TRAIL, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs));
@@ -1560,19 +1439,23 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
         }
         if (lv.small.cnt) {
             Timer t(h, K_SMALL);
-            // shared memory for the level's largest front (as FP64 up to
-            // kSmallRescue rows, for the in-place rescue of an FP32 front) and
-            // 128 threads for levels of many narrow fronts: more fronts in
-            // flight (a level of few fronts keeps 256 threads, for latency)
-            const int mj = lv.small_maxnj;
-            const int rj = std::min(mj, kSmallRescue);
-            const size_t sm = std::max<size_t>((size_t)mj * mj * sizeof(T), sizeof(T) == 4 ? (size_t)rj * rj * 8 : 0);
-            const bool wide = lv.small.cnt >= kSmallWideLevel;
-            const unsigned nt = !wide || mj > kSmallNarrowNJ ? 256 : mj <= kSmallTinyNJ ? 64 : 128;
-            launch_k(k_small<T, LDLT>, grid_for(lv.small.cnt), nt, sm, h->stream, 
-                h->d_fronts, items + lv.small.off, h->d_reltgt, h->d_chdtgt, fb.P, fb.M, fb.d, h->d_signs,
-                h->d_info, h->d_rescued, reg);
-            MF_CUDA(cudaGetLastError());
+            // one launch sized for the level's largest front; a level that
+            // fills the SMs several times over takes one launch per size
+            // class (a class of less than one front per SM joins the next)
+            int64_t off = lv.small.off, cnt = 0;
+            int stage = 0;
+            for (int c = 0; c < kSmallClasses; ++c) {
+                cnt += lv.small_cls[c];
+                stage = std::max(stage, lv.small_stage[c]);
+                const bool last = off + cnt == lv.small.off + lv.small.cnt;
+                if (!cnt || (!last && (lv.small.cnt < kSmallWideLevel || cnt < 148))) continue;
+                if (int rc = launch_small<T, LDLT, REG>(h, ItemList{off, cnt}, last ? lv.small_maxnj : kSmallClassNJ[c],
+                                                   stage, fb, reg))
+                    return rc;
+                off += cnt;
+                cnt = 0;
+                stage = 0;
+            }
         }
         if (lv.ea.cnt) {
             Timer t(h, K_EA);
@@ -1624,7 +1507,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
                 }
                 if (st.diag.cnt) {
                     Timer t(h, K_DIAG);
-                    launch_kx(h->panel_pdl || pdl_enabled(), k_diag<T, LDLT>, grid_for(st.diag.cnt), 256,
+                    launch_kx(h->panel_pdl || pdl_enabled(), k_diag<T, LDLT, REG>, grid_for(st.diag.cnt), 256,
                         diag_smem<T>(), h->stream, h->d_fronts, items + st.diag.off, c0, fb.P, fb.inv, fb.d,
                         h->d_signs, h->d_info, h->d_rescued, reg);
                     MF_CUDA(cudaGetLastError());
@@ -1660,7 +1543,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
             }
             if (st.diag.cnt) {
                 Timer t(h, K_DIAG);
-                launch_kx(h->panel_pdl || pdl_enabled(), k_diag<T, LDLT>, grid_for(st.diag.cnt), 256,
+                launch_kx(h->panel_pdl || pdl_enabled(), k_diag<T, LDLT, REG>, grid_for(st.diag.cnt), 256,
                     diag_smem<T>(), h->stream, h->d_fronts, items + st.diag.off, c0, fb.P, fb.inv, fb.d,
                     h->d_signs, h->d_info, h->d_rescued, reg);
                 MF_CUDA(cudaGetLastError());
@@ -1777,7 +1660,8 @@ int launch_factor(mf_handle* h) {
     }
     FactorBufs<double> fb{h->d_P, h->d_M, h->d_inv, h->d_d, h->d_inv2};
     int rc = run_captured(h, 1, (int64_t)(uintptr_t)h->d_signs, 0, 0, [&]() {
-        return h->diag ? factor_impl<double, 1>(h, fb) : factor_impl<double, 0>(h, fb);
+        if (h->reg.delta >= 0.0) return h->diag ? factor_impl<double, 1, true>(h, fb) : factor_impl<double, 0, true>(h, fb);
+        return h->diag ? factor_impl<double, 1, false>(h, fb) : factor_impl<double, 0, false>(h, fb);
     });
     h->fp64_current = rc == 0;
     h->selinv_done = false;
@@ -1791,7 +1675,7 @@ int launch_factor_mixed(mf_handle* h) {
         if (rc) return rc;
     }
     return run_captured(h, 2, (int64_t)(uintptr_t)h->d_signs, h->use_tc ? 1 : 0, 0, [&]() {
-        return h->diag ? factor_impl<float, 1>(h, fb) : factor_impl<float, 0>(h, fb);
+        return h->diag ? factor_impl<float, 1, false>(h, fb) : factor_impl<float, 0, false>(h, fb);
     });
 }
 

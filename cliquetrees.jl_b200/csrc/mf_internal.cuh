@@ -89,6 +89,11 @@ struct ItemList {
 constexpr int kSmallMax = 96;   // fronts with nj <= kSmallMax: one fused CTA
 constexpr int kWarpSmallNJ = 16; // of those, fronts with nj <= kWarpSmallNJ: one warp each (k_small_warp)
 constexpr int kWarpSmallNJ2 = 32; // and kWarpSmallNJ < nj <= kWarpSmallNJ2: one warp each, 32-row variant
+// k_small's size classes (largest nj each): 64-thread CTAs up to 48 rows, 256 above
+constexpr int kSmallClasses = 4;
+constexpr int kSmallClassNJ[kSmallClasses] = {32, 48, 64, kSmallMax};
+constexpr int kSmallStage = 96 * 96; // most entries of children a small front stages at once (its largest child fits)
+constexpr int kSmallWideLevel = 4 * 148;  // small fronts of a level from which it is split by size
 constexpr int kTinyNJ = 16;      // solves: fronts with nj <= kTinyNJ take 16 lanes each (k_s_tiny_*)
 constexpr int kTinyNJ2 = 32;     // and kTinyNJ < nj <= kTinyNJ2 a warp each, with k_s_tiny_*'s design
 constexpr int kNB = 64;         // sub-panel width of the blocked path
@@ -142,10 +147,12 @@ struct SolveStep {
 };
 
 struct Level {
-    ItemList small_warp;     // (front)           fronts with nj <= kWarpSmallNJ: one warp each (k_small_warp)
+    ItemList small_warp;     // (front)           fronts with nj <= kWarpSmallNJ on levels of many: one warp each (k_small_warp)
     ItemList small_warp2;    // (front)           kWarpSmallNJ < nj <= kWarpSmallNJ2: one warp each (MF_WARP_FRONT32=0: k_small)
     ItemList small;          // (front)           other fronts with nj <= kSmallMax: one CTA each (k_small)
     int small_maxnj = 0;     // largest nj of those (sizes k_small's shared memory and CTA)
+    int64_t small_cls[kSmallClasses] = {0};  // how many of them fall in each size class; the list is in class order
+    int small_stage[kSmallClasses] = {0};    // entries of children staged at once, per class (<= kSmallStage)
     // extend-add for blocked fronts, item (front, col tile, row chunk, first
     // segment): ea adds the children into the panel columns before the
     // panel is factored; ea_upd adds them into the update matrix after the

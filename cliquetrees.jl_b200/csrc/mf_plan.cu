@@ -417,10 +417,16 @@ int build_plan(mf_handle* h, const int64_t* resptr, const int64_t* sepptr, const
         Level& lv = h->levels[L];
         const std::vector<int32_t>& fr = by_level[L];
         // factorization
+        // fronts of at most kWarpSmallNJ rows take a warp each where there are
+        // enough of them to fill the SMs; fewer join the CTA-per-front list
+        // (a shorter chain per front, and one launch less)
+        int64_t nwarp = 0;
+        for (int32_t j : fr) nwarp += h->h_fronts[j].nn + h->h_fronts[j].na <= kWarpSmallNJ;
+        const int wmin = nwarp >= kSmallWideLevel ? kWarpSmallNJ : 0;  // largest nj of the warp list
         begin(lv.small_warp);
         for (int32_t j : fr) {
             const Front& f = h->h_fronts[j];
-            if (f.nn + f.na <= kWarpSmallNJ) push(j, 0, 0);
+            if (f.nn + f.na <= wmin) push(j, 0, 0);
         }
         end(lv.small_warp);
         begin(lv.small_warp2);
@@ -430,13 +436,25 @@ int build_plan(mf_handle* h, const int64_t* resptr, const int64_t* sepptr, const
         }
         end(lv.small_warp2);
         begin(lv.small);
-        for (int32_t j : fr) {
-            const Front& f = h->h_fronts[j];
-            if (f.nn + f.na > (warp32 ? kWarpSmallNJ2 : kWarpSmallNJ) && f.nn + f.na <= kSmallMax) {
+        for (int c = 0; c < kSmallClasses; ++c)
+            for (int32_t j : fr) {
+                const Front& f = h->h_fronts[j];
+                const int nj = f.nn + f.na;
+                if (nj <= wmin || (warp32 && nj > kWarpSmallNJ && nj <= kWarpSmallNJ2)) continue;
+                if (nj > kSmallClassNJ[c] || (c > 0 && nj <= kSmallClassNJ[c - 1])) continue;
                 push(j, 0, 0);
-                lv.small_maxnj = std::max(lv.small_maxnj, f.nn + f.na);
+                lv.small_cls[c] += 1;
+                lv.small_maxnj = std::max(lv.small_maxnj, nj);
+                // staged children: all of them where they fit the front's own
+                // size again, else as many as do (at least the largest)
+                int one = 0, all = 0;
+                for (int32_t p = f.chd0; p < f.chd1; ++p) {
+                    const Front& fc = h->h_fronts[(size_t)h->h_exec_chd[(size_t)p]];
+                    one = std::max(one, fc.ldm * fc.na);
+                    all = std::min(all + fc.ldm * fc.na, kSmallStage);
+                }
+                lv.small_stage[c] = std::max(lv.small_stage[c], std::max(one, std::min(all, f.ldp * nj)));
             }
-        }
         end(lv.small);
         int max_steps = 0;
         for (int part = 0; part < 2; ++part) {
