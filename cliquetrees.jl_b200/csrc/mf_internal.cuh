@@ -113,6 +113,12 @@ constexpr int kTcTrailN = 128;  // tile columns of the tensor-core trailing upda
 constexpr int kSplitRows = 128;  // rows of a pre-split operand unit
 constexpr int kSplitK = 32;      // columns (K) of a pre-split operand unit
 constexpr int kSplitUnitFloats = 2 * kSplitRows * kSplitK;  // hi and lo tiles: 32 KB
+// Small fronts of a level up to which each takes a CTA in the solves: eight per
+// SM, about what the SMs hold at once (a level then costs one front's latency,
+// 4 to 8 us against a warp's 10 to 20 us).  Above it warps (k_s_small_*,
+// k_s_tiny_*) keep more fronts in flight: 5 us for a level of 8,000 tiny ones.
+constexpr int kCtaFronts = 8 * 148;
+constexpr int kMaxSmem = 225 * 1024;  // dynamic shared memory a CTA may ask for beside its static part
 constexpr int kFwdRows = 64;    // rows per forward-update work item
 constexpr int kSolveNB = 256;   // columns of a solve step: a super-block of four 64-column diagonal blocks
 constexpr int kBwdRows = 512;   // rows of L21 per backward partial-sum work item
@@ -167,6 +173,13 @@ struct Level {
     ItemList syrk_tc;        // 128 x 64 tiles for the tcgen05 kernel
     ItemList split_syrk;     // (front, row block, chunk, first unit) of the SYRK's split operands
     // solves
+    // a level's small fronts: s_cta holds them all, a CTA each, where there are
+    // at most kCtaFronts (a chain of narrow levels waits for each front's
+    // latency); else s_small / s_tiny / s_tiny2 (wide levels: throughput)
+    ItemList s_cta;          // (front)
+    int s_cta_panel = 0;     // shared-memory entries of the largest panel: as stored,
+    int s_cta_pad32 = 0, s_cta_pad64 = 0;  // with the backward kernel's padded columns (FP32, FP64)
+    int s_cta_rows = 0;      // largest nj, odd
     ItemList s_small;        // (front)
     ItemList s_tiny;         // (front)           small fronts with nj <= kTinyNJ: 16 lanes each
     ItemList s_tiny2;        // (front)           small fronts with kTinyNJ < nj <= kTinyNJ2: a warp each
@@ -505,6 +518,9 @@ int launch_solve(mf_handle* h, int64_t nrhs);
 // (R: nrval_per_rhs*nrhs, W and C: n*nrhs, part: nbwd_part*64*16 doubles)
 int launch_solve_with(mf_handle* h, int64_t nrhs, double* R, double* W, double* C, double* part);
 int launch_solve_mixed(mf_handle* h, int64_t nrhs);
+// the small fronts of a narrow level (mf_solve_small.cu)
+int launch_solve_cta(mf_handle* h, const Level& lv, const SolveBufs<double>& sb, int bwd, int nrb, int nrhs);
+int launch_solve_cta(mf_handle* h, const Level& lv, const SolveBufs<float>& sb, int bwd, int nrb, int nrhs);
 int launch_permute_to(mf_handle* h, const double* B, int64_t ldb, const int64_t* perm, int64_t nrhs, double* dst);
 int launch_permute_from(mf_handle* h, double* B, int64_t ldb, const int64_t* perm, int64_t nrhs, const double* src);
 int launch_anorm(mf_handle* h);

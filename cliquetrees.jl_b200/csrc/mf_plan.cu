@@ -659,25 +659,35 @@ int build_plan(mf_handle* h, const int64_t* resptr, const int64_t* sepptr, const
 
         // solves: small fronts (solve_small) one warp each; blocked fronts in
         // 256-column super-block steps using the super-block inverses
-        begin(lv.s_small);
+        int64_t nsmall = 0;
+        for (int32_t j : fr) nsmall += solve_small(h->h_fronts[j]) && task_of[j] < 0;
+        const bool cta = nsmall <= kCtaFronts;
+        begin(lv.s_cta);
         for (int32_t j : fr) {
             const Front& f = h->h_fronts[j];
-            if (solve_small(f) && task_of[j] < 0 && f.nn + f.na > kTinyNJ2) push(j, 0, 0);
+            if (!cta || !solve_small(f) || task_of[j] >= 0) continue;
+            push(j, 0, 0);
+            // 16-byte units per column rounded up to an odd number (pad_ld)
+            const int u32 = (f.ldp / 4) | 1, u64 = (f.ldp / 2) | 1;
+            lv.s_cta_panel = std::max(lv.s_cta_panel, f.ldp * f.nn);
+            lv.s_cta_pad32 = std::max(lv.s_cta_pad32, 4 * u32 * f.nn);
+            lv.s_cta_pad64 = std::max(lv.s_cta_pad64, 2 * u64 * f.nn);
+            lv.s_cta_rows = std::max(lv.s_cta_rows, (f.nn + f.na) | 1);
         }
-        end(lv.s_small);
-        begin(lv.s_tiny);
-        for (int32_t j : fr) {
-            const Front& f = h->h_fronts[j];
-            if (solve_small(f) && task_of[j] < 0 && f.nn + f.na <= kTinyNJ) push(j, 0, 0);
-        }
-        end(lv.s_tiny);
-        begin(lv.s_tiny2);
-        for (int32_t j : fr) {
-            const Front& f = h->h_fronts[j];
-            const int nj = f.nn + f.na;
-            if (solve_small(f) && task_of[j] < 0 && nj > kTinyNJ && nj <= kTinyNJ2) push(j, 0, 0);
-        }
-        end(lv.s_tiny2);
+        end(lv.s_cta);
+        // (front) lists of a wide level, by size
+        auto sized = [&](ItemList& l, int lo, int hi) {
+            begin(l);
+            for (int32_t j : fr) {
+                const Front& f = h->h_fronts[j];
+                const int nj = f.nn + f.na;
+                if (!cta && solve_small(f) && task_of[j] < 0 && nj > lo && nj <= hi) push(j, 0, 0);
+            }
+            end(l);
+        };
+        sized(lv.s_small, kTinyNJ2, INT32_MAX);
+        sized(lv.s_tiny, 0, kTinyNJ);
+        sized(lv.s_tiny2, kTinyNJ, kTinyNJ2);
         // forward gather: item (front, row tile, first row pointer of the
         // front, 0).  Row q of a blocked front owns the list of the children's
         // update rows that land on it, children in reverse order (the order

@@ -1752,6 +1752,8 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
     }
     // forward: levels ascending
     for (const Level& lv : h->levels) {
+        if (lv.s_cta.cnt)
+            if (int rc = launch_solve_cta(h, lv, sb, 0, nrb, nrhs)) return rc;
         if (lv.s_tiny.cnt)
             if (int rc = launch_tiny<T, UNIT, 0, kTinyNJ>(h, lv.s_tiny, sb, nrb, nrhs)) return rc;
         if (lv.s_tiny2.cnt)
@@ -1897,6 +1899,8 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
                 MF_CUDA(cudaGetLastError());
             }
         }
+        if (lv.s_cta.cnt)
+            if (int rc = launch_solve_cta(h, lv, sb, 1, nrb, nrhs)) return rc;
         if (lv.s_small.cnt) {
             Timer t(h, K_S_SMALL);
             const unsigned g = (unsigned)((lv.s_small.cnt + kSmallWarps - 1) / kSmallWarps);
