@@ -17,8 +17,8 @@
 //               diagonal block in shared memory, writes it back and stores
 //               the inverse of the factored block (potrf! of chol_factor!,
 //               cholesky.jl:694-737);
-//   k_gemm    : grouped 64x64 DMMA (mma.sync m8n8k4 f64) tile GEMM with a
-//               cp.async double-buffered K loop, in four roles: left-looking
+//   k_gemm64  : grouped DMMA (mma.sync m8n8k4 f64) tile GEMM, 128 x 64 or
+//               64 x 64 tiles (FP32: mf_tc.cu, or k_gemm), in four roles: left-looking
 //               update of a sub-panel from its outer block, trailing update
 //               of the panel after an outer block (K = 256), the TRSM of a
 //               sub-panel as a product with the inverse of its diagonal
@@ -946,12 +946,11 @@ __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ front
 }
 
 // ---------------------------------------------------------------------------
-// Tile GEMM with a cp.async double-buffered K loop:
+// FP32 tile GEMM without tensor cores (the autotuner's alternative to mf_tc.cu's
+// tiles on levels of small fronts), with a cp.async double-buffered K loop:
 // acc(64x64) += A(64 x K) * B(64 x K)^T.  Shared tiles are [k][m] with m
-// contiguous (leading dimension LDS).
-//   double: DMMA (mma.sync m8n8k4 f64), 8 warps; warp w owns rows
-//           (w&1)*32..+32 and columns (w>>1)*16..+16 as 4 x 2 fragments.
-//   float : FMA, thread t owns rows (t>>4)*4..+4 and columns (t&15)*4..+4.
+// contiguous (leading dimension LDS); thread t owns rows (t>>4)*4..+4 and
+// columns (t&15)*4..+4.
 // ---------------------------------------------------------------------------
 constexpr int KC = 32;                   // K chunk per pipeline stage
 constexpr int STAGE = KC * LDS;          // elements per matrix per stage
@@ -962,20 +961,10 @@ constexpr int gemm_smem() { return (4 * STAGE + 2 * KC) * (int)sizeof(T); }
 template <typename T>
 struct Acc;
 template <>
-struct Acc<double> {
-    double c[4][2][2];
-};
-template <>
 struct Acc<float> {
     float c[4][4];
 };
 
-__device__ __forceinline__ void acc_zero(Acc<double>& a) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) a.c[i][j][0] = a.c[i][j][1] = 0.0;
-}
 __device__ __forceinline__ void acc_zero(Acc<float>& a) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -1007,25 +996,6 @@ __device__ __forceinline__ void stage_chunk(T* As, T* Bs, const T* A, int64_t ld
         const T* sb = B + (vb ? (rb + m) + (int64_t)(k + kk) * ldb : 0);
         cp_async_el(As + m + kk * LDS, sa, va);
         cp_async_el(Bs + m + kk * LDS, sb, vb);
-    }
-}
-
-__device__ __forceinline__ void mma_chunk(Acc<double>& acc, const double* As, const double* Bs, const double* dsc,
-                                          int kc) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wr = (warp & 1) * 32, wc = (warp >> 1) * 16;
-    const int fr = lane >> 2, fk = lane & 3;
-    for (int k = 0; k < kc; k += 4) {
-        double a[4], b[2];
-        const double s = dsc ? dsc[k + fk] : 1.0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = As[(wr + i * 8 + fr) + (k + fk) * LDS] * s;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) b[j] = Bs[(wc + j * 8 + fr) + (k + fk) * LDS];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) dmma(acc.c[i][j][0], acc.c[i][j][1], a[i], b[j]);
     }
 }
 
@@ -1079,18 +1049,6 @@ __device__ void gemm_k_loop(Acc<T>& acc, T* smem, const T* A, int64_t lda, int r
 }
 
 // visit every accumulator element as (row, col, value)
-template <typename F>
-__device__ __forceinline__ void acc_for_each(const Acc<double>& acc, F&& fn) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wr = (warp & 1) * 32, wc = (warp >> 1) * 16;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-                fn(wr + i * 8 + (lane >> 2), wc + j * 8 + (lane & 3) * 2 + e, acc.c[i][j][e]);
-}
 template <typename F>
 __device__ __forceinline__ void acc_for_each(const Acc<float>& acc, F&& fn) {
     const int tr = (threadIdx.x >> 4) * 4, tc = (threadIdx.x & 15) * 4;
@@ -1161,6 +1119,203 @@ __global__ void __launch_bounds__(256) k_gemm(const Front* __restrict__ fronts, 
             __syncthreads();
         }
         acc_store<1>(acc, Pj + (int64_t)c0 * ld, ld, rs, 0, nj - rs, w, false, LDLT ? (const T*)sc : nullptr);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 tile GEMM of the blocked fronts: acc(BM x 64) = A(BM x K) B(64 x K)^T on
+// DMMA (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind), a warp per 32 x 32.
+//   BM = 128, 8 warps: sixteen independent products per four k and eight
+//     shared-memory reads for them, two CTAs per SM, so one CTA's prologue and
+//     C update hide behind the other's products;
+//   BM = 64, 4 warps: launches of few tiles, where the SMs would idle.
+// What bounds the large launches is the FP64 pipe (64 FMA a cycle and SM:
+// 36.9 TFLOP/s measured for DMMA alone); 80^3: SYRKs 40.7 -> 36.5 ms, trailing
+// updates 23.1 -> 20.6, left updates 5.9 -> 4.2, KKT 24 left updates 1.56 ->
+// 1.01 ms, against 64 x 64 tiles of eight warps fed by 8-byte copies, two
+// barriers per 32 k. operands come in 16-byte asynchronous copies, three
+// stages of 16 k deep, one barrier a stage.  Tiles are columns of the panel
+// (rows contiguous, [k][row] in shared memory with 4 doubles of padding: a
+// fragment read touches every bank once).  A copy needs an even row start;
+// tiles on an odd row (a 64-row SYRK tile of an odd nn) copy 8 bytes at a time.
+// ---------------------------------------------------------------------------
+constexpr int GK = 16, GStages = 3;
+template <int BM>
+constexpr int g64_stage() { return GK * (BM + 4) + GK * (kTile + 4) + GK; }  // A, B, pivots (doubles)
+template <int BM>
+constexpr int g64_smem() { return GStages * g64_stage<BM>() * (int)sizeof(double); }
+template <int BM>
+constexpr int g64_threads() { return 32 * (BM / 32) * (kTile / 32); }
+
+// copy rows [row0, row0 + ROWS) x columns [k, k + GK) of a column-major matrix
+// into dst[kk * (ROWS + 4) + m]; rows at or past rlim (rounded up to the next
+// even one) and columns at or past kend become zeros
+template <int ROWS, int NT, bool VEC>
+__device__ __forceinline__ void g64_copy(double* dst, const double* src, int64_t ld, int row0, int rlim, int k, int kend) {
+    constexpr int W = VEC ? 2 : 1, PER = ROWS / W;
+    static_assert((GK * PER) % NT == 0, "whole rounds of copies");
+#pragma unroll
+    for (int u = 0; u < GK * PER / NT; ++u) {
+        const int i = threadIdx.x + u * NT;
+        const int m = (i % PER) * W, kk = i / PER;
+        const bool ok = row0 + m < rlim && k + kk < kend;
+        const double* s = src + (ok ? (row0 + m) + (int64_t)(k + kk) * ld : 0);
+        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + kk * (ROWS + 4) + m);
+        if (VEC)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(s), "r"(ok ? 16 : 0) : "memory");
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(s), "r"(ok ? 8 : 0) : "memory");
+    }
+}
+
+// Items of BM = 64 are the (front, 64-row tile, 64-column tile) lists; of
+// BM = 128 the tensor-core lists (128-row tiles, 128-column ones for the
+// trailing update and the SYRK, which start on 4-row boundaries), two CTAs an
+// item there: column half blockIdx & 1.
+template <int BM, int ROLE, int LDLT>
+__global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64(const Front* __restrict__ fronts,
+                                                                 const Item* __restrict__ items, int obs, int obw,
+                                                                 int c0, double* __restrict__ P,
+                                                                 double* __restrict__ M, const double* __restrict__ d,
+                                                                 const double* __restrict__ inv) {
+    pdl_prologue();
+    constexpr int NT = g64_threads<BM>(), LA = BM + 4, LB = kTile + 4, STG = g64_stage<BM>();
+    constexpr bool PAIR = BM == 128 && (ROLE == G_TRAIL || ROLE == G_SYRK);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* smem = reinterpret_cast<double*>(smem_raw);
+    const Item it = items[PAIR ? blockIdx.x >> 1 : blockIdx.x];
+    const int half = PAIR ? (int)(blockIdx.x & 1) * kTile : 0;
+    const Front f = fronts[it.front];
+    const int nn = f.nn, na = f.na, nj = nn + na, ld = f.ldp;
+    double* Pj = P + f.poff;
+    // panel rows ra.. (A) and rb.. (B) over columns [kbeg, kend); C rows
+    // [rlo, rhi) x columns [clo, chi) in panel coordinates, at C + row + col * ldc
+    int ra, rb, kbeg, kend, rlo, rhi = nj, clo, chi, blim = nj;
+    const double* Bm = Pj;
+    int64_t ldb = ld, ldc = ld;
+    double* C = Pj;
+    bool tri = true;
+    if (ROLE == G_LEFT) {
+        ra = c0 + it.a * BM, rb = c0, kbeg = obs, kend = c0;
+        rlo = clo = c0, chi = min(nn, c0 + kNB);
+    } else if (ROLE == G_TRAIL) {
+        const int e = min(nn, obs + obw);
+        const int cs = e + it.b * (PAIR ? 2 * kTile : kTile);
+        ra = cs + it.a * BM, rb = cs + half, kbeg = obs, kend = e;
+        rlo = clo = e, chi = nn;
+    } else if (ROLE == G_SYRK) {
+        const int x0 = PAIR ? nn & ~3 : nn;
+        // 64-row tiles: item (row tile, column tile); 128-row ones: (row tile below the diagonal, column tile)
+        ra = PAIR ? x0 + it.b * 2 * kTile + it.a * BM : x0 + it.a * BM;
+        rb = x0 + it.b * (PAIR ? 2 * kTile : kTile) + half;
+        kbeg = 0, kend = nn, rlo = clo = nn, chi = nj;
+        C = M + f.moff - nn - (int64_t)nn * f.ldm;
+        ldc = f.ldm;
+    } else {
+        const int r0 = min(nn, c0 + kNB);
+        ra = (BM == 128 ? r0 & ~3 : r0) + it.a * BM, rb = 0, kbeg = c0, kend = r0;
+        rlo = r0, clo = c0, chi = r0;
+        Bm = inv + f.ioff + (int64_t)(c0 / kNB) * kNB * kNB - (int64_t)c0 * kNB;
+        ldb = kNB, blim = kNB, tri = false;
+    }
+    if (tri && ra + BM <= rb) return;  // wholly above the diagonal
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wr = (warp % (BM / 32)) * 32, wc = (warp / (BM / 32)) * 32;
+    const int fr = lane >> 2, fk = lane & 3;
+    const double* dj = (LDLT && ROLE != G_TRSM) ? d + f.col0 : nullptr;
+    const bool vec = ((ra | rb) & 1) == 0;
+    const int nchunk = (kend - kbeg + GK - 1) / GK;
+    auto load = [&](int c) {
+        if (c < nchunk) {
+            double* st = smem + (c % GStages) * STG;
+            const int k = kbeg + c * GK;
+            if (vec) {
+                g64_copy<BM, NT, true>(st, Pj, ld, ra, nj, k, kend);
+                g64_copy<kTile, NT, true>(st + GK * LA, Bm, ldb, rb, blim, k, kend);
+            } else {
+                g64_copy<BM, NT, false>(st, Pj, ld, ra, nj, k, kend);
+                g64_copy<kTile, NT, false>(st + GK * LA, Bm, ldb, rb, blim, k, kend);
+            }
+            if (LDLT && ROLE != G_TRSM && tid < GK) {
+                const bool ok = k + tid < kend;
+                const unsigned sd = (unsigned)__cvta_generic_to_shared(st + GK * (LA + LB) + tid);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sd), "l"(dj + (ok ? k + tid : 0)),
+                             "r"(ok ? 8 : 0)
+                             : "memory");
+            }
+        }
+        cp_commit();
+    };
+    double acc[4][4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+#pragma unroll
+    for (int c = 0; c < GStages - 1; ++c) load(c);
+    double rd[4][2];  // TRSM of LDLt: reciprocal pivots of the thread's columns, formed beside the copies
+    if (LDLT && ROLE == G_TRSM)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int col = c0 + wc + j * 8 + fk * 2 + e;
+                rd[j][e] = col < chi ? 1.0 / d[f.col0 + col] : 1.0;
+            }
+    for (int c = 0; c < nchunk; ++c) {
+        cp_wait<GStages - 2>();
+        __syncthreads();
+        load(c + GStages - 1);  // into the stage that every warp finished before this barrier
+        const double* As = smem + (c % GStages) * STG;
+        const double* Bs = As + GK * LA;
+        const double* Ds = Bs + GK * LB;
+#pragma unroll
+        for (int k = 0; k < GK; k += 4) {
+            double a[4], b[4];
+            const double s = (LDLT && ROLE != G_TRSM) ? Ds[k + fk] : 1.0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                a[i] = As[(k + fk) * LA + wr + i * 8 + fr];
+                if (LDLT && ROLE != G_TRSM) a[i] *= s;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = Bs[(k + fk) * LB + wc + j * 8 + fr];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+        }
+    }
+    // C = -acc (SYRK), acc / d (TRSM) or C - acc: eight columns' worth of C is
+    // read before the first of it is written
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int row = ra + wr + i * 8 + fr;
+        const bool rok = row >= rlo && row < rhi;
+        double cv[4][2];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int col = (ROLE == G_TRSM ? c0 : rb) + wc + j * 8 + fk * 2 + e;
+                const bool ok = rok && col >= clo && col < chi && (!tri || row >= col);
+                cv[j][e] = (ok && (ROLE == G_LEFT || ROLE == G_TRAIL)) ? C[row + (int64_t)col * ldc] : 0.0;
+            }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int col = (ROLE == G_TRSM ? c0 : rb) + wc + j * 8 + fk * 2 + e;
+                const bool ok = rok && col >= clo && col < chi && (!tri || row >= col);
+                if (!ok) continue;
+                double v = acc[i][j][e];
+                if (ROLE == G_TRSM) {
+                    if (LDLT) v *= rd[j][e];
+                } else {
+                    v = cv[j][e] - v;
+                }
+                C[row + (int64_t)col * ldc] = v;
+            }
     }
 }
 
@@ -1368,6 +1523,46 @@ int launch_panel32_to_dl(mf_handle* h, double* dD, double* dL) {
 }
 
 
+// one role of the FP64 factorization: 128-row tiles when they give every SM at
+// least two CTAs, else 64-row ones (a launch of fewer large tiles leaves SMs
+// idle for a whole tile's time)
+template <int ROLE, int LDLT>
+static int gemm64(mf_handle* h, const ItemList& small, const ItemList& large, int obs, int obw, int c0,
+                  const FactorBufs<double>& fb) {
+    if (!small.cnt) return 0;
+    constexpr bool PAIR = ROLE == G_TRAIL || ROLE == G_SYRK;
+    const int64_t big = large.cnt * (PAIR ? 2 : 1);
+    const bool pdl = pdl_enabled() || (h->panel_pdl && !PAIR);
+    if (big >= 2 * (int64_t)(h->num_sms > 0 ? h->num_sms : 148)) {
+        MF_CUDA(cudaFuncSetAttribute(k_gemm64<128, ROLE, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, g64_smem<128>()));
+        launch_kx(pdl, k_gemm64<128, ROLE, LDLT>, grid_for(big), g64_threads<128>(), g64_smem<128>(), h->stream,
+                  h->d_fronts, h->d_items + large.off, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
+    } else {
+        MF_CUDA(cudaFuncSetAttribute(k_gemm64<64, ROLE, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, g64_smem<64>()));
+        launch_kx(pdl, k_gemm64<64, ROLE, LDLT>, grid_for(small.cnt), g64_threads<64>(), g64_smem<64>(), h->stream,
+                  h->d_fronts, h->d_items + small.off, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
+    }
+    MF_CUDA(cudaGetLastError());
+    return 0;
+}
+
+// one role of a level's panel steps or SYRK without the tcgen05 tiles
+template <typename T, int ROLE, int LDLT>
+static int gemm_role(mf_handle* h, const ItemList& small, const ItemList& large, int obs, int obw, int c0,
+                     const FactorBufs<T>& fb) {
+    if constexpr (std::is_same<T, double>::value) {
+        return gemm64<ROLE, LDLT>(h, small, large, obs, obw, c0, fb);
+    } else {
+        constexpr int gs = gemm_smem<T>();
+        MF_CUDA(cudaFuncSetAttribute(k_gemm<T, ROLE, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs));
+        launch_kx(pdl_enabled() || (h->panel_pdl && (ROLE == G_LEFT || ROLE == G_TRSM)), k_gemm<T, ROLE, LDLT>,
+                  grid_for(small.cnt), 256, gs, h->stream, h->d_fronts, h->d_items + small.off, obs, obw, c0, fb.P, fb.M,
+                  fb.d, fb.inv);
+        MF_CUDA(cudaGetLastError());
+        return 0;
+    }
+}
+
 // k_small over one run of a level's small fronts of at most mj rows: 64
 // threads up to 48 rows (two warps keep the barriers of the pivot chain
 // short), 256 above.  Shared memory holds `stage` staged
@@ -1399,17 +1594,12 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
     // the pivot rule applies to the FP64 factorization; the mixed form keeps
     // NoRegularization (its single-precision factor only preconditions)
     const Reg reg = std::is_same<T, double>::value ? h->reg : Reg();
-    constexpr int gs = gemm_smem<T>();
     MF_CUDA(cudaFuncSetAttribute(k_small_warp<T, LDLT, kWarpSmallNJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kWarpFronts * warp_slice<kWarpSmallNJ>()));
     MF_CUDA(cudaFuncSetAttribute(k_small_warp<T, LDLT, kWarpSmallNJ2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kWarpFronts * warp_slice<kWarpSmallNJ2>()));
     MF_CUDA(cudaFuncSetAttribute(k_diag<T, LDLT, REG>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<T>()));
     MF_CUDA(cudaFuncSetAttribute(k_inv256<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, inv256_smem<T>()));
-    MF_CUDA(cudaFuncSetAttribute(k_gemm<T, G_LEFT, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs));
-    MF_CUDA(cudaFuncSetAttribute(k_gemm<T, G_TRAIL, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs));
-    MF_CUDA(cudaFuncSetAttribute(k_gemm<T, G_SYRK, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs));
-    MF_CUDA(cudaFuncSetAttribute(k_gemm<T, G_TRSM, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs));
     const Item* items = h->d_items;
     // per-level timing while autotuning (profile mode: no graph, synchronised)
     cudaEvent_t tev[3] = {nullptr, nullptr, nullptr};
@@ -1537,9 +1727,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
             }
             if (st.left.cnt) {
                 Timer t(h, K_LEFT);
-                launch_kx(h->panel_pdl || pdl_enabled(), k_gemm<T, G_LEFT, LDLT>, grid_for(st.left.cnt), 256, gs,
-                    h->stream, h->d_fronts, items + st.left.off, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
-                MF_CUDA(cudaGetLastError());
+                if (int rc = gemm_role<T, G_LEFT, LDLT>(h, st.left, st.left_tc, obs, obw, c0, fb)) return rc;
             }
             if (st.diag.cnt) {
                 Timer t(h, K_DIAG);
@@ -1550,24 +1738,21 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
             }
             if (st.panel.cnt) {
                 Timer t(h, K_PANEL);
-                launch_kx(h->panel_pdl || pdl_enabled(), k_gemm<T, G_TRSM, LDLT>, grid_for(st.panel.cnt), 256, gs,
-                    h->stream, h->d_fronts, items + st.panel.off, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
-                MF_CUDA(cudaGetLastError());
+                if (int rc = gemm_role<T, G_TRSM, LDLT>(h, st.panel, st.panel_tc, obs, obw, c0, fb)) return rc;
             }
             if (st.trail.cnt) {
                 Timer t(h, K_UPDATE);
                 if (int rc = join()) return rc;
                 const bool la = la_on && st.trail_ncrit > 0 && st.trail_ncrit < st.trail.cnt;
-                const int64_t ncrit = la ? st.trail_ncrit : st.trail.cnt;
-                launch_k(k_gemm<T, G_TRAIL, LDLT>, grid_for(ncrit), 256, gs, h->stream,
-                    h->d_fronts, items + st.trail.off, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
-                MF_CUDA(cudaGetLastError());
+                const int64_t n1 = la ? st.trail_ncrit : st.trail.cnt, n2 = la ? st.trail_tc_ncrit : st.trail_tc.cnt;
+                if (int rc = gemm_role<T, G_TRAIL, LDLT>(h, ItemList{st.trail.off, n1}, ItemList{st.trail_tc.off, n2}, obs,
+                                                         obw, c0, fb))
+                    return rc;
                 if (la) {
                     const int rc = on_side([&]() -> int {
-                        launch_k(k_gemm<T, G_TRAIL, LDLT>, grid_for(st.trail.cnt - ncrit), 256, gs, h->stream,
-                            h->d_fronts, items + st.trail.off + ncrit, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
-                        MF_CUDA(cudaGetLastError());
-                        return 0;
+                        return gemm_role<T, G_TRAIL, LDLT>(h, ItemList{st.trail.off + n1, st.trail.cnt - n1},
+                                                           ItemList{st.trail_tc.off + n2, st.trail_tc.cnt - n2}, obs, obw,
+                                                           c0, fb);
                     });
                     if (rc) return rc;
                 }
@@ -1585,9 +1770,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
             }
         } else if (lv.syrk.cnt) {
             Timer t(h, K_SYRK);
-            launch_k(k_gemm<T, G_SYRK, LDLT>, grid_for(lv.syrk.cnt), 256, gs, h->stream, 
-                h->d_fronts, items + lv.syrk.off, 0, 0, 0, fb.P, fb.M, fb.d, fb.inv);
-            MF_CUDA(cudaGetLastError());
+            if (int rc = gemm_role<T, G_SYRK, LDLT>(h, lv.syrk, lv.syrk_tc, 0, 0, 0, fb)) return rc;
         }
         if (lv.ea_upd.cnt) {
             Timer t(h, K_EA);
