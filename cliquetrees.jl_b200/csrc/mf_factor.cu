@@ -1124,11 +1124,15 @@ __global__ void __launch_bounds__(256) k_gemm(const Front* __restrict__ fronts, 
 
 // ---------------------------------------------------------------------------
 // FP64 tile GEMM of the blocked fronts: acc(BM x 64) = A(BM x K) B(64 x K)^T on
-// DMMA (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind), a warp per 32 x 32.
+// DMMA (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind), a warp per 32 x 32
+// (16 x 32 for BM = 32).
 //   BM = 128, 8 warps: sixteen independent products per four k and eight
 //     shared-memory reads for them, two CTAs per SM, so one CTA's prologue and
 //     C update hide behind the other's products;
-//   BM = 64, 4 warps: launches of few tiles, where the SMs would idle.
+//   BM = 64, 4 warps: launches of few tiles, where the SMs would idle;
+//   BM = 32, 4 warps, two CTAs a 64-row item: launches of fewer 64-row tiles
+//     than SMs, which last as long as one tile's products (KKT 24: 12.26 ->
+//     11.75 ms a pass, 100^2 922 -> 886 us).
 // What bounds the large launches is the FP64 pipe (64 FMA a cycle and SM:
 // 36.9 TFLOP/s measured for DMMA alone); 80^3: SYRKs 40.7 -> 36.5 ms, trailing
 // updates 23.1 -> 20.6, left updates 5.9 -> 4.2, KKT 24 left updates 1.56 ->
@@ -1145,7 +1149,9 @@ constexpr int g64_stage() { return GK * (BM + 4) + GK * (kTile + 4) + GK; }  // 
 template <int BM>
 constexpr int g64_smem() { return GStages * g64_stage<BM>() * (int)sizeof(double); }
 template <int BM>
-constexpr int g64_threads() { return 32 * (BM / 32) * (kTile / 32); }
+constexpr int g64_wm() { return BM == 32 ? 16 : 32; }  // rows per warp
+template <int BM>
+constexpr int g64_threads() { return 32 * (BM / g64_wm<BM>()) * (kTile / 32); }
 
 // copy rows [row0, row0 + ROWS) x columns [k, k + GK) of a column-major matrix
 // into dst[kk * (ROWS + 4) + m]; rows at or past rlim (rounded up to the next
@@ -1168,7 +1174,7 @@ __device__ __forceinline__ void g64_copy(double* dst, const double* src, int64_t
     }
 }
 
-// Items of BM = 64 are the (front, 64-row tile, 64-column tile) lists; of
+// Items of BM <= 64 are the (front, 64-row tile, 64-column tile) lists; of
 // BM = 128 the tensor-core lists (128-row tiles, 128-column ones for the
 // trailing update and the SYRK, which start on 4-row boundaries), two CTAs an
 // item there: column half blockIdx & 1.
@@ -1183,11 +1189,13 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
     constexpr bool PAIR = BM == 128 && (ROLE == G_TRAIL || ROLE == G_SYRK);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* smem = reinterpret_cast<double*>(smem_raw);
-    const Item it = items[PAIR ? blockIdx.x >> 1 : blockIdx.x];
+    constexpr int IR = BM == 32 ? kTile : BM;  // rows of an item
+    const Item it = items[(PAIR || BM == 32) ? blockIdx.x >> 1 : blockIdx.x];
     const int half = PAIR ? (int)(blockIdx.x & 1) * kTile : 0;
     const Front f = fronts[it.front];
     const int nn = f.nn, na = f.na, nj = nn + na, ld = f.ldp;
     double* Pj = P + f.poff;
+    const int row0 = it.a * IR + (BM == 32 ? (int)(blockIdx.x & 1) * BM : 0);
     // panel rows ra.. (A) and rb.. (B) over columns [kbeg, kend); C rows
     // [rlo, rhi) x columns [clo, chi) in panel coordinates, at C + row + col * ldc
     int ra, rb, kbeg, kend, rlo, rhi = nj, clo, chi, blim = nj;
@@ -1196,31 +1204,32 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
     double* C = Pj;
     bool tri = true;
     if (ROLE == G_LEFT) {
-        ra = c0 + it.a * BM, rb = c0, kbeg = obs, kend = c0;
+        ra = c0 + row0, rb = c0, kbeg = obs, kend = c0;
         rlo = clo = c0, chi = min(nn, c0 + kNB);
     } else if (ROLE == G_TRAIL) {
         const int e = min(nn, obs + obw);
         const int cs = e + it.b * (PAIR ? 2 * kTile : kTile);
-        ra = cs + it.a * BM, rb = cs + half, kbeg = obs, kend = e;
+        ra = cs + row0, rb = cs + half, kbeg = obs, kend = e;
         rlo = clo = e, chi = nn;
     } else if (ROLE == G_SYRK) {
         const int x0 = PAIR ? nn & ~3 : nn;
         // 64-row tiles: item (row tile, column tile); 128-row ones: (row tile below the diagonal, column tile)
-        ra = PAIR ? x0 + it.b * 2 * kTile + it.a * BM : x0 + it.a * BM;
+        ra = PAIR ? x0 + it.b * 2 * kTile + row0 : x0 + row0;
         rb = x0 + it.b * (PAIR ? 2 * kTile : kTile) + half;
         kbeg = 0, kend = nn, rlo = clo = nn, chi = nj;
         C = M + f.moff - nn - (int64_t)nn * f.ldm;
         ldc = f.ldm;
     } else {
         const int r0 = min(nn, c0 + kNB);
-        ra = (BM == 128 ? r0 & ~3 : r0) + it.a * BM, rb = 0, kbeg = c0, kend = r0;
+        ra = (BM == 128 ? r0 & ~3 : r0) + row0, rb = 0, kbeg = c0, kend = r0;
         rlo = r0, clo = c0, chi = r0;
         Bm = inv + f.ioff + (int64_t)(c0 / kNB) * kNB * kNB - (int64_t)c0 * kNB;
         ldb = kNB, blim = kNB, tri = false;
     }
-    if (tri && ra + BM <= rb) return;  // wholly above the diagonal
+    if (ra >= rhi || (tri && ra + BM <= rb)) return;  // past the rows, or wholly above the diagonal
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wr = (warp % (BM / 32)) * 32, wc = (warp / (BM / 32)) * 32;
+    constexpr int WM = g64_wm<BM>(), MI = WM / 8;
+    const int wr = (warp % (BM / WM)) * WM, wc = (warp / (BM / WM)) * 32;
     const int fr = lane >> 2, fk = lane & 3;
     const double* dj = (LDLT && ROLE != G_TRSM) ? d + f.col0 : nullptr;
     const bool vec = ((ra | rb) & 1) == 0;
@@ -1246,9 +1255,9 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
         }
         cp_commit();
     };
-    double acc[4][4][2];
+    double acc[MI][4][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll
@@ -1271,17 +1280,17 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
         const double* Ds = Bs + GK * LB;
 #pragma unroll
         for (int k = 0; k < GK; k += 4) {
-            double a[4], b[4];
+            double a[MI], b[4];
             const double s = (LDLT && ROLE != G_TRSM) ? Ds[k + fk] : 1.0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < MI; ++i) {
                 a[i] = As[(k + fk) * LA + wr + i * 8 + fr];
                 if (LDLT && ROLE != G_TRSM) a[i] *= s;
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) b[j] = Bs[(k + fk) * LB + wc + j * 8 + fr];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < MI; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
         }
@@ -1289,7 +1298,7 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
     // C = -acc (SYRK), acc / d (TRSM) or C - acc: eight columns' worth of C is
     // read before the first of it is written
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < MI; ++i) {
         const int row = ra + wr + i * 8 + fr;
         const bool rok = row >= rlo && row < rhi;
         double cv[4][2];
@@ -1523,27 +1532,30 @@ int launch_panel32_to_dl(mf_handle* h, double* dD, double* dL) {
 }
 
 
+template <int BM, int ROLE, int LDLT>
+static int gemm64_go(mf_handle* h, int64_t ctas, const Item* items, int obs, int obw, int c0,
+                     const FactorBufs<double>& fb) {
+    const bool pdl = pdl_enabled() || (h->panel_pdl && (ROLE == G_LEFT || ROLE == G_TRSM));
+    MF_CUDA(cudaFuncSetAttribute(k_gemm64<BM, ROLE, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, g64_smem<BM>()));
+    launch_kx(pdl, k_gemm64<BM, ROLE, LDLT>, grid_for(ctas), g64_threads<BM>(), g64_smem<BM>(), h->stream, h->d_fronts,
+              items, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
+    MF_CUDA(cudaGetLastError());
+    return 0;
+}
+
 // one role of the FP64 factorization: 128-row tiles when they give every SM at
 // least two CTAs, else 64-row ones (a launch of fewer large tiles leaves SMs
-// idle for a whole tile's time)
+// idle for a whole tile's time), 32-row ones when even those are fewer than
+// the SMs
 template <int ROLE, int LDLT>
 static int gemm64(mf_handle* h, const ItemList& small, const ItemList& large, int obs, int obw, int c0,
                   const FactorBufs<double>& fb) {
     if (!small.cnt) return 0;
-    constexpr bool PAIR = ROLE == G_TRAIL || ROLE == G_SYRK;
-    const int64_t big = large.cnt * (PAIR ? 2 : 1);
-    const bool pdl = pdl_enabled() || (h->panel_pdl && !PAIR);
-    if (big >= 2 * (int64_t)(h->num_sms > 0 ? h->num_sms : 148)) {
-        MF_CUDA(cudaFuncSetAttribute(k_gemm64<128, ROLE, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, g64_smem<128>()));
-        launch_kx(pdl, k_gemm64<128, ROLE, LDLT>, grid_for(big), g64_threads<128>(), g64_smem<128>(), h->stream,
-                  h->d_fronts, h->d_items + large.off, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
-    } else {
-        MF_CUDA(cudaFuncSetAttribute(k_gemm64<64, ROLE, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, g64_smem<64>()));
-        launch_kx(pdl, k_gemm64<64, ROLE, LDLT>, grid_for(small.cnt), g64_threads<64>(), g64_smem<64>(), h->stream,
-                  h->d_fronts, h->d_items + small.off, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
-    }
-    MF_CUDA(cudaGetLastError());
-    return 0;
+    const int64_t big = large.cnt * (ROLE == G_TRAIL || ROLE == G_SYRK ? 2 : 1), sms = h->num_sms > 0 ? h->num_sms : 148;
+    const Item* items = h->d_items;
+    if (big >= 2 * sms) return gemm64_go<128, ROLE, LDLT>(h, big, items + large.off, obs, obw, c0, fb);
+    if (small.cnt >= sms) return gemm64_go<64, ROLE, LDLT>(h, small.cnt, items + small.off, obs, obw, c0, fb);
+    return gemm64_go<32, ROLE, LDLT>(h, 2 * small.cnt, items + small.off, obs, obw, c0, fb);
 }
 
 // one role of a level's panel steps or SYRK without the tcgen05 tiles
