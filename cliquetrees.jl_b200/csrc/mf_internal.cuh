@@ -152,6 +152,14 @@ struct SolveStep {
     ItemList bwd;     // (front, col tile)  columns left of the super-block -= L^T x_K
 };
 
+// small fronts that take a CTA each in the solves (mf_solve_small.cu)
+struct CtaList {
+    ItemList items;            // (front)
+    int panel = 0;             // shared-memory entries of the largest panel: as stored,
+    int pad32 = 0, pad64 = 0;  // with the backward kernel's padded columns (FP32, FP64)
+    int rows = 0;              // largest nj, odd
+};
+
 struct Level {
     ItemList small_warp;     // (front)           fronts with nj <= kWarpSmallNJ on levels of many: one warp each (k_small_warp)
     ItemList small_warp2;    // (front)           kWarpSmallNJ < nj <= kWarpSmallNJ2: one warp each (MF_WARP_FRONT32=0: k_small)
@@ -176,10 +184,7 @@ struct Level {
     // a level's small fronts: s_cta holds them all, a CTA each, where there are
     // at most kCtaFronts (a chain of narrow levels waits for each front's
     // latency); else s_small / s_tiny / s_tiny2 (wide levels: throughput)
-    ItemList s_cta;          // (front)
-    int s_cta_panel = 0;     // shared-memory entries of the largest panel: as stored,
-    int s_cta_pad32 = 0, s_cta_pad64 = 0;  // with the backward kernel's padded columns (FP32, FP64)
-    int s_cta_rows = 0;      // largest nj, odd
+    CtaList s_cta;
     ItemList s_small;        // (front)
     ItemList s_tiny;         // (front)           small fronts with nj <= kTinyNJ: 16 lanes each
     ItemList s_tiny2;        // (front)           small fronts with kTinyNJ < nj <= kTinyNJ2: a warp each

@@ -662,19 +662,20 @@ int build_plan(mf_handle* h, const int64_t* resptr, const int64_t* sepptr, const
         int64_t nsmall = 0;
         for (int32_t j : fr) nsmall += solve_small(h->h_fronts[j]) && task_of[j] < 0;
         const bool cta = nsmall <= kCtaFronts;
-        begin(lv.s_cta);
+        CtaList& cl = lv.s_cta;
+        begin(cl.items);
         for (int32_t j : fr) {
             const Front& f = h->h_fronts[j];
             if (!cta || !solve_small(f) || task_of[j] >= 0) continue;
             push(j, 0, 0);
             // 16-byte units per column rounded up to an odd number (pad_ld)
             const int u32 = (f.ldp / 4) | 1, u64 = (f.ldp / 2) | 1;
-            lv.s_cta_panel = std::max(lv.s_cta_panel, f.ldp * f.nn);
-            lv.s_cta_pad32 = std::max(lv.s_cta_pad32, 4 * u32 * f.nn);
-            lv.s_cta_pad64 = std::max(lv.s_cta_pad64, 2 * u64 * f.nn);
-            lv.s_cta_rows = std::max(lv.s_cta_rows, (f.nn + f.na) | 1);
+            cl.panel = std::max(cl.panel, f.ldp * f.nn);
+            cl.pad32 = std::max(cl.pad32, 4 * u32 * f.nn);
+            cl.pad64 = std::max(cl.pad64, 2 * u64 * f.nn);
+            cl.rows = std::max(cl.rows, (f.nn + f.na) | 1);
         }
-        end(lv.s_cta);
+        end(cl.items);
         // (front) lists of a wide level, by size
         auto sized = [&](ItemList& l, int lo, int hi) {
             begin(l);
@@ -859,7 +860,8 @@ int build_plan(mf_handle* h, const int64_t* resptr, const int64_t* sepptr, const
             const int rows = f.nn + f.na - (f.nn & ~3);
             const int nchunk = (int)cdiv(f.nn, kFwdCols);
             for (int t = 0; t < (int)cdiv(rows, kFwdRows); ++t) {
-                fred.push_back(Item{j, t, fslot, nchunk});
+                // (a front of one chunk needs no reduction: k_s_fwd_l takes its sums from R)
+                if (nchunk > 1) fred.push_back(Item{j, t, fslot, nchunk});
                 for (int q = 0; q < nchunk; ++q) items.push_back(Item{j, t, q, fslot++});
             }
         }
@@ -878,7 +880,7 @@ int build_plan(mf_handle* h, const int64_t* resptr, const int64_t* sepptr, const
             bfirst.push_back(slot);
             const int nchunk = std::max<int>(1, (int)cdiv(f.na, kBwdRows));
             for (int t = 0; t < cdiv(f.nn, kNB); ++t) {
-                red.push_back(Item{j, t, slot, 0});
+                if (nchunk > 1) red.push_back(Item{j, t, slot, 0});  // one chunk: k_s_bwd_l forms W itself
                 for (int q = 0; q < nchunk; ++q) items.push_back(Item{j, t, q, slot++});
             }
         }

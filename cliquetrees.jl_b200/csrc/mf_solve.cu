@@ -13,6 +13,8 @@
 // (na x nrhs, ld na) and are pulled by the parent.  In the backward pass the
 // reference pushes F restricted to sep(i) to each child; that vector is the
 // already-final solution at rows sep(i), so children read it from C directly.
+#include <type_traits>
+
 #include "mf_internal.cuh"
 
 namespace mf {
@@ -630,36 +632,51 @@ __global__ void __launch_bounds__(kSubWarps * 32, small_min_blocks<T, NR>() / 2)
 // row's own list of child contributions (h_grow / h_gcon, children in the
 // reference's order), so no two threads touch one entry and the tile needs
 // no barrier
-template <typename T>
+// wait(): taken once the lists (static) are at hand, before the vectors are read
+struct GatherNoWait {
+    __device__ void operator()() const {}
+};
+struct GatherPdlWait {
+    __device__ void operator()() const { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+};
+template <typename T, typename Wait = GatherNoWait>
 __device__ __forceinline__ void gather_run(const Item& it, const Front* __restrict__ fronts,
                                            const int64_t* __restrict__ grow, const GCon* __restrict__ gcon,
-                                           const T* __restrict__ C, T* W, T* R, int64_t n, int nrhs) {
+                                           const T* C, T* W, T* R, int64_t n, int nrhs, Wait wait = Wait()) {
     const Front f = fronts[it.front];
     const int nn = f.nn, na = f.na, nj = nn + na;
     const int p0 = it.a * kSolveRows, p1 = min(p0 + kSolveRows, nj);
     const int w = p1 - p0;
     const int64_t* rp = grow + it.b;
     T* Rj = R + f.roff * nrhs;
+    int64_t e0 = 0, e1 = 0;
+    GCon g{};
+    bool waited = false;
     for (int i = threadIdx.x; i < w * nrhs; i += blockDim.x) {
         const int q = p0 + i % w, r = i / w;
+        e0 = rp[q], e1 = rp[q + 1];
+        if (e0 < e1) g = gcon[e0];
+        if (!waited) wait();
+        waited = true;
         T v = q < nn ? C[f.col0 + q + (int64_t)r * n] : T(0);
-        const int64_t e1 = rp[q + 1];
-        for (int64_t e = rp[q]; e < e1; ++e) {
-            const GCon g = gcon[e];
-            v += R[g.roff * nrhs + g.a + (int64_t)r * g.ma];
+        for (int64_t e = e0; e < e1; ++e) {
+            const GCon c = g;
+            if (e + 1 < e1) g = gcon[e + 1];
+            v += R[c.roff * nrhs + c.a + (int64_t)r * c.ma];
         }
         if (q < nn) W[f.col0 + q + (int64_t)r * n] = v;
         else Rj[(q - nn) + (int64_t)r * na] = v;
     }
+    if (!waited) wait();
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_s_gather(const Front* __restrict__ fronts, const Item* __restrict__ items,
                                                   const int64_t* __restrict__ grow,
-                                                  const GCon* __restrict__ gcon, const T* __restrict__ C,
-                                                  T* __restrict__ W, T* __restrict__ R, int64_t n, int nrhs) {
-    pdl_prologue();
-    gather_run<T>(items[blockIdx.x], fronts, grow, gcon, C, W, R, n, nrhs);
+                                                  const GCon* __restrict__ gcon, const T* C, T* W, T* R, int64_t n,
+                                                  int nrhs) {
+    pdl_trigger();
+    gather_run<T>(items[blockIdx.x], fronts, grow, gcon, C, W, R, n, nrhs, GatherPdlWait());
 }
 
 // ---------------------------------------------------------------------------
@@ -942,14 +959,23 @@ __global__ void __launch_bounds__(256) k_s_ftile(const Front* __restrict__ front
 // and the chunk's sums for the tile's rows go to part[slot]; k_s_fwd_red adds
 // the chunks of a tile in order.  This takes the L21 product (most of the
 // forward data of a large front) out of the sequential step chain.
+// whether the L21 products start beside the grid before them and load their
+// first panel entries ahead of the wait for the level's vectors: a level of few
+// items waits for memory (512^2 FP32, four right-hand sides: 10.0 -> 8.3 us a
+// backward launch, 7.9 -> 6.2 forward); with wide vectors (48^3 FP64, eight)
+// staging those is what takes the time, and it cost 25.7 -> 31.3 us
+template <typename T, int NR>
+constexpr bool early_panel() { return NR * (int)sizeof(T) <= 16; }
+
 template <typename T, int NR>
 constexpr int fwdl_smem() { return (kFwdCols * NR + 8 * NR * kFwdRows) * (int)sizeof(T); }
 
 template <typename T, int NR>
 __global__ void __launch_bounds__(256) k_s_fwd_l(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                                 const T* __restrict__ P, const T* __restrict__ C,
-                                                 T* __restrict__ part, int64_t n, int nrhs) {
-    pdl_prologue();
+                                                 const T* __restrict__ P, const T* C, T* part, T* R,
+                                                 int64_t n, int nrhs) {
+    if (early_panel<T, NR>()) pdl_trigger();
+    else pdl_prologue();
     using VT = Vec16<T>;
     using V = typename VT::type;
     constexpr int VW = VT::W;             // rows per load
@@ -964,11 +990,6 @@ __global__ void __launch_bounds__(256) k_s_fwd_l(const Front* __restrict__ front
     const int cq = it.b * kFwdCols, wq = min(kFwdCols, nn - cq);
     const int ra = (nn & ~3) + it.a * kFwdRows;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < kFwdCols * NR; i += 256) {
-        const int c = i % kFwdCols, r = i / kFwdCols;
-        xs[c * NR + r] = (c < wq && r < nrhs) ? C[f.col0 + cq + c + (int64_t)r * n] : T(0);
-    }
-    __syncthreads();
     const int rr = (lane % LPC) * VW, ch = lane / LPC;
     // row is a multiple of 4 below nj, so the 16-byte load ends inside the
     // column's ldp (a multiple of 4) rows
@@ -980,17 +1001,37 @@ __global__ void __launch_bounds__(256) k_s_fwd_l(const Front* __restrict__ front
     for (int e = 0; e < VW; ++e)
 #pragma unroll
         for (int r = 0; r < NR; ++r) acc[e][r] = T(0);
-    if (row < nj && cn > 0) {
-        const T* pc = P + f.poff + (int64_t)(cq + cb) * ld + row;
-        // all of a batch's loads are issued before its products (one
-        // memory round trip per 16 columns of a lane, in column order)
-        for (int cb0 = ch; cb0 < cn; cb0 += kColBatchL * CPL) {
-            V lb[kColBatchL];
+    const bool act = row < nj && cn > 0;
+    const T* pc = P + f.poff + (int64_t)(cq + cb) * ld + row;
+    V lb[kColBatchL];
+    auto first = [&]() {
+        if (act)
 #pragma unroll
             for (int u = 0; u < kColBatchL; ++u) {
-                const int c = cb0 + u * CPL;
+                const int c = ch + u * CPL;
                 if (c < cn) lb[u] = *reinterpret_cast<const V*>(pc + (int64_t)c * ld);
             }
+    };
+    if (early_panel<T, NR>()) {
+        first();
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+    for (int i = tid; i < kFwdCols * NR; i += 256) {
+        const int c = i % kFwdCols, r = i / kFwdCols;
+        xs[c * NR + r] = (c < wq && r < nrhs) ? C[f.col0 + cq + c + (int64_t)r * n] : T(0);
+    }
+    __syncthreads();
+    if (!early_panel<T, NR>()) first();
+    if (act) {
+        // all of a batch's loads are issued before its products (one
+        // memory round trip per batch of a lane's columns, in column order)
+        for (int cb0 = ch; cb0 < cn; cb0 += kColBatchL * CPL) {
+            if (cb0 != ch)
+#pragma unroll
+                for (int u = 0; u < kColBatchL; ++u) {
+                    const int c = cb0 + u * CPL;
+                    if (c < cn) lb[u] = *reinterpret_cast<const V*>(pc + (int64_t)c * ld);
+                }
 #pragma unroll
             for (int u = 0; u < kColBatchL; ++u) {
                 const int c = cb0 + u * CPL;
@@ -1019,21 +1060,26 @@ __global__ void __launch_bounds__(256) k_s_fwd_l(const Front* __restrict__ front
             for (int e = 0; e < VW; ++e) red[(warp * NR + r) * kFwdRows + rr + e] = acc[e][r];
     }
     __syncthreads();
+    // a front of one column chunk subtracts its sums from R_j itself
+    const bool one = nn <= kFwdCols;
     T* dst = part + (int64_t)it.pad * (kFwdRows * kMaxRhs);
-    for (int o = tid; o < kFwdRows * kMaxRhs; o += 256) {
+    T* Rj = R + f.roff * nrhs;
+    for (int o = tid; o < kFwdRows * (one ? NR : kMaxRhs); o += 256) {
         const int rl = o % kFwdRows, r = o / kFwdRows;
         T v = T(0);
         if (r < NR)
 #pragma unroll
             for (int w = 0; w < 8; ++w) v += red[(w * NR + r) * kFwdRows + rl];
-        dst[o] = v;
+        const int q = ra + rl;
+        if (!one) dst[o] = v;
+        else if (r < nrhs && q >= nn && q < nj) Rj[(q - nn) + r * f.na] -= v;
     }
 }
 
 // R_j[rows of tile t] -= the chunk sums of k_s_fwd_l, chunks in order.
 template <typename T>
 __global__ void __launch_bounds__(256) k_s_fwd_red(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                                   const T* __restrict__ part, T* __restrict__ R, int nrhs) {
+                                                   const T* part, T* R, int nrhs) {
     pdl_prologue();
     const Item it = items[blockIdx.x];
     const Front f = fronts[it.front];
@@ -1273,12 +1319,14 @@ template <typename T, int NR>
 constexpr int bwd_smem() { return (kBwdAlignRows * NR + 4 * NR * kNB) * (int)sizeof(T); }
 
 // one work item (front f, 64-column tile it.a, row chunk it.b, slot it.pad);
+// DIRECT: a front of one row chunk forms W[tile] = C - sum itself; wait() is
+// taken after the first loads of the panel;
 // BATCH 16-byte loads of a thread are in flight at once (the order of the
 // products does not depend on it)
-template <typename T, int NR, int BATCH>
+template <typename T, int NR, int BATCH, bool DIRECT = false, typename Wait = GatherNoWait>
 __device__ __forceinline__ void bwdl_run(const Front& f, const Item& it, const int32_t* __restrict__ septgt,
-                                         const T* __restrict__ P, const T* __restrict__ C, T* part, int64_t n,
-                                         int nrhs, unsigned char* sm_raw) {
+                                         const T* __restrict__ P, const T* C, T* part, int64_t n,
+                                         int nrhs, unsigned char* sm_raw, T* W = nullptr, Wait wait = Wait()) {
     using VT = Vec16<T>;
     using V = typename VT::type;
     constexpr int VW = VT::W;
@@ -1292,27 +1340,38 @@ __device__ __forceinline__ void bwdl_run(const Front& f, const Item& it, const i
     const int rlo = nn + a_beg, rhi = nn + a_end;  // panel rows of the chunk
     const int row0 = rlo & ~3;                     // 4-aligned start of the staged rows
     const int nrow = rhi - row0;                   // <= kBwdAlignRows
-    for (int i = tid; i < kBwdAlignRows * NR; i += 256) {
-        const int a = i % kBwdAlignRows, r = i / kBwdAlignRows;
-        const int row = row0 + a;
-        xs[a * NR + r] = (row >= rlo && row < rhi && r < nrhs) ? C[sep[row - nn] + (int64_t)r * n] : T(0);
-    }
-    __syncthreads();
     const int c = tid & (kNB - 1), q = tid >> 6;
     constexpr int QR = kBwdAlignRows / 4;      // rows per quarter (a multiple of 4)
     const int i0 = q * QR, ni = min(QR, nrow - i0);
     T acc[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) acc[r] = T(0);
-    if (c < wc && ni > 0) {
-        // row0 + i0 + i is a multiple of 4 below rhi <= nj, so each 16-byte
-        // load ends inside the column's ldp rows
-        const T* pc = P + f.poff + (int64_t)(c0 + c) * ld + row0 + i0;
-        for (int i = 0; i < QR; i += BATCH * VW) {
-            V l[BATCH];
+    // row0 + i0 + i is a multiple of 4 below rhi <= nj, so each 16-byte
+    // load ends inside the column's ldp rows
+    const T* pc = P + f.poff + (int64_t)(c0 + c) * ld + row0 + i0;
+    const bool act = c < wc && ni > 0;
+    V l[BATCH];
+    auto first = [&]() {
+        if (act)
 #pragma unroll
             for (int u = 0; u < BATCH; ++u)
-                if (i + u * VW < ni) l[u] = *reinterpret_cast<const V*>(pc + i + u * VW);
+                if (u * VW < ni) l[u] = *reinterpret_cast<const V*>(pc + u * VW);
+    };
+    if (early_panel<T, NR>()) first();
+    wait();
+    for (int i = tid; i < kBwdAlignRows * NR; i += 256) {
+        const int a = i % kBwdAlignRows, r = i / kBwdAlignRows;
+        const int row = row0 + a;
+        xs[a * NR + r] = (row >= rlo && row < rhi && r < nrhs) ? C[sep[row - nn] + (int64_t)r * n] : T(0);
+    }
+    __syncthreads();
+    if (!early_panel<T, NR>()) first();
+    if (act) {
+        for (int i = 0; i < QR; i += BATCH * VW) {
+            if (i != 0)
+#pragma unroll
+                for (int u = 0; u < BATCH; ++u)
+                    if (i + u * VW < ni) l[u] = *reinterpret_cast<const V*>(pc + i + u * VW);
 #pragma unroll
             for (int u = 0; u < BATCH; ++u) {
                 const int ib = i + u * VW;
@@ -1333,34 +1392,41 @@ __device__ __forceinline__ void bwdl_run(const Front& f, const Item& it, const i
 #pragma unroll
     for (int r = 0; r < NR; ++r) red[(q * NR + r) * kNB + c] = acc[r];
     __syncthreads();
+    const bool one = DIRECT && na <= kBwdRows;
     T* dst = part + (int64_t)it.pad * (kNB * kMaxRhs);
-    for (int o = tid; o < kNB * kMaxRhs; o += 256) {
+    for (int o = tid; o < kNB * (one ? NR : kMaxRhs); o += 256) {
         const int cc = o % kNB, r = o / kNB;
         T v = T(0);
         if (r < NR)
             v = red[(0 * NR + r) * kNB + cc] + red[(1 * NR + r) * kNB + cc] + red[(2 * NR + r) * kNB + cc] +
                 red[(3 * NR + r) * kNB + cc];
-        dst[o] = v;
+        if (!one) {
+            dst[o] = v;
+        } else if (cc < wc && r < nrhs) {
+            const int64_t idx = f.col0 + c0 + cc + (int64_t)r * n;
+            W[idx] = C[idx] - v;
+        }
     }
 }
 
 template <typename T, int NR>
 __global__ void __launch_bounds__(256) k_s_bwd_l(const Front* __restrict__ fronts, const Item* __restrict__ items,
                                                  const int32_t* __restrict__ septgt, const T* __restrict__ P,
-                                                 const T* __restrict__ C, T* __restrict__ part, int64_t n,
-                                                 int nrhs) {
-    pdl_prologue();
+                                                 const T* C, T* part, T* W, int64_t n, int nrhs) {
+    if (early_panel<T, NR>()) pdl_trigger();
+    else pdl_prologue();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     const Item it = items[blockIdx.x];
     const Front f = fronts[it.front];
-    bwdl_run<T, NR, kColBatchL>(f, it, septgt, P, C, part, n, nrhs, sm_raw);
+    using Wait = typename std::conditional<early_panel<T, NR>(), GatherPdlWait, GatherNoWait>::type;
+    bwdl_run<T, NR, kColBatchL, true>(f, it, septgt, P, C, part, n, nrhs, sm_raw, W, Wait());
 }
 
 // W[tile it.a of the front's columns] = C - (the chunk sums at part[it.b ...],
 // chunks in order); part is read through L2 (in k_s_mid_bwd other CTAs of
 // the cluster wrote it)
 template <typename T>
-__device__ __forceinline__ void bwdred_run(const Front& f, const Item& it, const T* part, const T* __restrict__ C,
+__device__ __forceinline__ void bwdred_run(const Front& f, const Item& it, const T* part, const T* C,
                                            T* W, int64_t n, int nrhs) {
     const int c0 = it.a * kNB, wc = min(kNB, f.nn - c0);
     const int nchunk = (f.na + kBwdRows - 1) / kBwdRows;
@@ -1376,8 +1442,7 @@ __device__ __forceinline__ void bwdred_run(const Front& f, const Item& it, const
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_s_bwd_red(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                                   const T* __restrict__ part, const T* __restrict__ C,
-                                                   T* __restrict__ W, int64_t n, int nrhs) {
+                                                   const T* part, const T* C, T* W, int64_t n, int nrhs) {
     pdl_prologue();
     const Item it = items[blockIdx.x];
     bwdred_run<T>(fronts[it.front], it, part, C, W, n, nrhs);
@@ -1752,7 +1817,7 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
     }
     // forward: levels ascending
     for (const Level& lv : h->levels) {
-        if (lv.s_cta.cnt)
+        if (lv.s_cta.items.cnt)
             if (int rc = launch_solve_cta(h, lv, sb, 0, nrb, nrhs)) return rc;
         if (lv.s_tiny.cnt)
             if (int rc = launch_tiny<T, UNIT, 0, kTinyNJ>(h, lv.s_tiny, sb, nrb, nrhs)) return rc;
@@ -1785,7 +1850,7 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
         }
         if (lv.s_gather.cnt) {
             Timer t(h, K_S_GATHER);
-            launch_k(k_s_gather<T>, (unsigned)lv.s_gather.cnt, 256, 0, h->stream, 
+            launch_kx(h->step_pdl, k_s_gather<T>, (unsigned)lv.s_gather.cnt, 256, 0, h->stream, 
                 h->d_fronts, items + lv.s_gather.off, h->d_grow, h->d_gcon, sb.C, sb.W, sb.R, n, nrhs);
             MF_CUDA(cudaGetLastError());
         }
@@ -1826,14 +1891,14 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
             const unsigned gl = (unsigned)lv.s_fwd_l.cnt;
             const Item* itl = items + lv.s_fwd_l.off;
             switch (nrb) {
-                case 1: launch_k(k_s_fwd_l<T, 1>, gl, 256, fwdl_smem<T, 1>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, n, nrhs); break;
-                case 2: launch_k(k_s_fwd_l<T, 2>, gl, 256, fwdl_smem<T, 2>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, n, nrhs); break;
-                case 4: launch_k(k_s_fwd_l<T, 4>, gl, 256, fwdl_smem<T, 4>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, n, nrhs); break;
-                case 8: launch_k(k_s_fwd_l<T, 8>, gl, 256, fwdl_smem<T, 8>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, n, nrhs); break;
-                default: launch_k(k_s_fwd_l<T, 16>, gl, 256, fwdl_smem<T, 16>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, n, nrhs); break;
+                case 1: launch_kx(early_panel<T, 1>() && h->step_pdl, k_s_fwd_l<T, 1>, gl, 256, fwdl_smem<T, 1>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
+                case 2: launch_kx(early_panel<T, 2>() && h->step_pdl, k_s_fwd_l<T, 2>, gl, 256, fwdl_smem<T, 2>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
+                case 4: launch_kx(early_panel<T, 4>() && h->step_pdl, k_s_fwd_l<T, 4>, gl, 256, fwdl_smem<T, 4>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
+                case 8: launch_kx(early_panel<T, 8>() && h->step_pdl, k_s_fwd_l<T, 8>, gl, 256, fwdl_smem<T, 8>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
+                default: launch_kx(early_panel<T, 16>() && h->step_pdl, k_s_fwd_l<T, 16>, gl, 256, fwdl_smem<T, 16>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
             }
             MF_CUDA(cudaGetLastError());
-            launch_k(k_s_fwd_red<T>, (unsigned)lv.s_fwd_red.cnt, 256, 0, h->stream, h->d_fronts, items + lv.s_fwd_red.off,
+            if (lv.s_fwd_red.cnt) launch_kx(h->step_pdl, k_s_fwd_red<T>, (unsigned)lv.s_fwd_red.cnt, 256, 0, h->stream, h->d_fronts, items + lv.s_fwd_red.off,
                                                                               sb.part, sb.R, nrhs);
             MF_CUDA(cudaGetLastError());
         }
@@ -1856,14 +1921,14 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
             const unsigned gl = (unsigned)lv.s_bwd_l.cnt;
             const Item* itl = items + lv.s_bwd_l.off;
             switch (nrb) {
-                case 1: launch_k(k_s_bwd_l<T, 1>, gl, 256, bwd_smem<T, 1>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, n, nrhs); break;
-                case 2: launch_k(k_s_bwd_l<T, 2>, gl, 256, bwd_smem<T, 2>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, n, nrhs); break;
-                case 4: launch_k(k_s_bwd_l<T, 4>, gl, 256, bwd_smem<T, 4>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, n, nrhs); break;
-                case 8: launch_k(k_s_bwd_l<T, 8>, gl, 256, bwd_smem<T, 8>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, n, nrhs); break;
-                default: launch_k(k_s_bwd_l<T, 16>, gl, 256, bwd_smem<T, 16>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, n, nrhs); break;
+                case 1: launch_kx(early_panel<T, 1>() && h->step_pdl, k_s_bwd_l<T, 1>, gl, 256, bwd_smem<T, 1>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 2: launch_kx(early_panel<T, 2>() && h->step_pdl, k_s_bwd_l<T, 2>, gl, 256, bwd_smem<T, 2>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 4: launch_kx(early_panel<T, 4>() && h->step_pdl, k_s_bwd_l<T, 4>, gl, 256, bwd_smem<T, 4>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 8: launch_kx(early_panel<T, 8>() && h->step_pdl, k_s_bwd_l<T, 8>, gl, 256, bwd_smem<T, 8>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                default: launch_kx(early_panel<T, 16>() && h->step_pdl, k_s_bwd_l<T, 16>, gl, 256, bwd_smem<T, 16>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
             }
             MF_CUDA(cudaGetLastError());
-            launch_k(k_s_bwd_red<T>, (unsigned)lv.s_bwd_red.cnt, 256, 0, h->stream, h->d_fronts, items + lv.s_bwd_red.off,
+            if (lv.s_bwd_red.cnt) launch_kx(h->step_pdl, k_s_bwd_red<T>, (unsigned)lv.s_bwd_red.cnt, 256, 0, h->stream, h->d_fronts, items + lv.s_bwd_red.off,
                                                                               sb.part, sb.C, sb.W, n, nrhs);
             MF_CUDA(cudaGetLastError());
         }
@@ -1899,7 +1964,7 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
                 MF_CUDA(cudaGetLastError());
             }
         }
-        if (lv.s_cta.cnt)
+        if (lv.s_cta.items.cnt)
             if (int rc = launch_solve_cta(h, lv, sb, 1, nrb, nrhs)) return rc;
         if (lv.s_small.cnt) {
             Timer t(h, K_S_SMALL);

@@ -45,9 +45,14 @@ __host__ __device__ constexpr int pad_ld(int ldp) {
     return ((ldp * (int)sizeof(T) / 16) & 1) ? ldp : ldp + 16 / (int)sizeof(T);
 }
 
-// right-hand sides a warp (column chain) or a thread (products) takes at once
+// right-hand sides a warp takes at once in the column chain
 template <int NR>
 constexpr int rhs_per_warp() { return NR > kCtaWarps ? NR / kCtaWarps : 1; }
+
+// right-hand sides a thread takes at once in the products with L21: few, so that
+// the rows (columns) of a small front times the groups fill the CTA
+template <int NR>
+constexpr int rhs_per_thread() { return NR >= 8 ? 4 : NR >= 4 ? 2 : 1; }
 
 // The triangular solve of one front by the CTA, vectors V[k + r * ldv] in
 // shared memory, L(i, k) at L[i * ri + k * rk]: forward (BWD = 0) columns
@@ -192,7 +197,7 @@ __global__ void __launch_bounds__(kCtaThreads) k_s_cta_fwd(const Front* __restri
     column_chain<T, UNIT, NR, 0>(Ps, ld, rinv, V, ldv, nn, nrhs, Cj, n);
     __syncthreads();
     // R_j = (child sums) - L21 x, a thread per row and group of right-hand sides
-    constexpr int Q = NR < 4 ? NR : 4, G = NR / Q;
+    constexpr int Q = rhs_per_thread<NR>(), G = NR / Q;
     T* Rj = R + f.roff * nrhs;
     for (int i = tid; i < na * G; i += kCtaThreads) {
         const int a = i % na, r0 = (i / na) * Q;
@@ -240,24 +245,31 @@ __global__ void __launch_bounds__(kCtaThreads) k_s_cta_bwd(const Front* __restri
     if (!UNIT)
         for (int k = tid; k < nn; k += kCtaThreads) rinv[k] = T(1) / Ps[k + k * ld];
     // C1 - L21^T x[sep]: a thread per column and group of right-hand sides,
-    // rows in order, 16 bytes of the column at a time from the aligned row at
-    // or before nn (rows before it are dropped)
-    constexpr int Q = NR < 4 ? NR : 4, G = NR / Q;
+    // rows in order, 16 bytes of the column at a time
+    constexpr int Q = rhs_per_thread<NR>(), G = NR / Q;
     for (int i = tid; i < nn * G; i += kCtaThreads) {
         const int k = i % nn, r0 = (i / nn) * Q;
         const T* l = Ps + k * ld;
+        const T* v = V + r0 * ldv;
         T acc[Q];
 #pragma unroll
         for (int r = 0; r < Q; ++r) acc[r] = T(0);
-        for (int a0 = nn & ~(W - 1); a0 < nj; a0 += W) {
+        int a0 = nn;
+        for (; (a0 & (W - 1)) && a0 < nj; ++a0)  // up to the first aligned row
+#pragma unroll
+            for (int r = 0; r < Q; ++r) acc[r] += l[a0] * v[a0 + r * ldv];
+#pragma unroll 2
+        for (; a0 + W <= nj; a0 += W) {
             T lv[W];
             *reinterpret_cast<int4*>(lv) = *reinterpret_cast<const int4*>(l + a0);
 #pragma unroll
             for (int e = 0; e < W; ++e)
-                if (a0 + e >= nn && a0 + e < nj)
 #pragma unroll
-                    for (int r = 0; r < Q; ++r) acc[r] += lv[e] * V[a0 + e + (r0 + r) * ldv];
+                for (int r = 0; r < Q; ++r) acc[r] += lv[e] * v[a0 + e + r * ldv];
         }
+        for (; a0 < nj; ++a0)
+#pragma unroll
+            for (int r = 0; r < Q; ++r) acc[r] += l[a0] * v[a0 + r * ldv];
 #pragma unroll
         for (int r = 0; r < Q; ++r) V[k + (r0 + r) * ldv] -= acc[r];
     }
@@ -266,43 +278,43 @@ __global__ void __launch_bounds__(kCtaThreads) k_s_cta_bwd(const Front* __restri
 }
 
 template <typename T, int UNIT, int NR>
-int cta_go(mf_handle* h, const Level& lv, const SolveBufs<T>& sb, int bwd, int nrhs) {
-    const Item* it = h->d_items + lv.s_cta.off;
-    const unsigned g = (unsigned)lv.s_cta.cnt;
-    const int pan = bwd ? (sizeof(T) == 4 ? lv.s_cta_pad32 : lv.s_cta_pad64) : lv.s_cta_panel;
-    const size_t sm = ((size_t)pan + (size_t)lv.s_cta_rows * NR + kSmallMax) * sizeof(T);
+int cta_go(mf_handle* h, const CtaList& l, const SolveBufs<T>& sb, int bwd, int nrhs) {
+    const Item* it = h->d_items + l.items.off;
+    const unsigned g = (unsigned)l.items.cnt;
+    const int pan = bwd ? (sizeof(T) == 4 ? l.pad32 : l.pad64) : l.panel;
+    const size_t sm = ((size_t)pan + (size_t)l.rows * NR + kSmallMax) * sizeof(T);
     if (!bwd) {
         MF_CUDA(cudaFuncSetAttribute(k_s_cta_fwd<T, UNIT, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
         launch_kx(h->step_pdl, k_s_cta_fwd<T, UNIT, NR>, g, kCtaThreads, sm, h->stream, h->d_fronts, it, pan,
-                  lv.s_cta_rows, h->d_reltgt, h->d_chdtgt, sb.P, sb.C, sb.R, h->n, nrhs);
+                  l.rows, h->d_reltgt, h->d_chdtgt, sb.P, sb.C, sb.R, h->n, nrhs);
     } else {
         MF_CUDA(cudaFuncSetAttribute(k_s_cta_bwd<T, UNIT, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
         launch_kx(h->step_pdl, k_s_cta_bwd<T, UNIT, NR>, g, kCtaThreads, sm, h->stream, h->d_fronts, it, pan,
-                  lv.s_cta_rows, h->d_septgt, sb.P, sb.C, h->n, nrhs);
+                  l.rows, h->d_septgt, sb.P, sb.C, h->n, nrhs);
     }
     MF_CUDA(cudaGetLastError());
     return 0;
 }
 
 template <typename T, int UNIT>
-int cta_rhs(mf_handle* h, const Level& lv, const SolveBufs<T>& sb, int bwd, int nrb, int nrhs) {
+int cta_rhs(mf_handle* h, const CtaList& l, const SolveBufs<T>& sb, int bwd, int nrb, int nrhs) {
     Timer t(h, K_S_SMALL);
     switch (nrb) {
-        case 1: return cta_go<T, UNIT, 1>(h, lv, sb, bwd, nrhs);
-        case 2: return cta_go<T, UNIT, 2>(h, lv, sb, bwd, nrhs);
-        case 4: return cta_go<T, UNIT, 4>(h, lv, sb, bwd, nrhs);
-        case 8: return cta_go<T, UNIT, 8>(h, lv, sb, bwd, nrhs);
-        default: return cta_go<T, UNIT, 16>(h, lv, sb, bwd, nrhs);
+        case 1: return cta_go<T, UNIT, 1>(h, l, sb, bwd, nrhs);
+        case 2: return cta_go<T, UNIT, 2>(h, l, sb, bwd, nrhs);
+        case 4: return cta_go<T, UNIT, 4>(h, l, sb, bwd, nrhs);
+        case 8: return cta_go<T, UNIT, 8>(h, l, sb, bwd, nrhs);
+        default: return cta_go<T, UNIT, 16>(h, l, sb, bwd, nrhs);
     }
 }
 
 }  // namespace
 
 int launch_solve_cta(mf_handle* h, const Level& lv, const SolveBufs<double>& sb, int bwd, int nrb, int nrhs) {
-    return h->diag ? cta_rhs<double, 1>(h, lv, sb, bwd, nrb, nrhs) : cta_rhs<double, 0>(h, lv, sb, bwd, nrb, nrhs);
+    return h->diag ? cta_rhs<double, 1>(h, lv.s_cta, sb, bwd, nrb, nrhs) : cta_rhs<double, 0>(h, lv.s_cta, sb, bwd, nrb, nrhs);
 }
 int launch_solve_cta(mf_handle* h, const Level& lv, const SolveBufs<float>& sb, int bwd, int nrb, int nrhs) {
-    return h->diag ? cta_rhs<float, 1>(h, lv, sb, bwd, nrb, nrhs) : cta_rhs<float, 0>(h, lv, sb, bwd, nrb, nrhs);
+    return h->diag ? cta_rhs<float, 1>(h, lv.s_cta, sb, bwd, nrb, nrhs) : cta_rhs<float, 0>(h, lv.s_cta, sb, bwd, nrb, nrhs);
 }
 
 }  // namespace mf
