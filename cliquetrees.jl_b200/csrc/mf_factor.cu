@@ -1332,103 +1332,151 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
 // 256x256 diagonal super-block inverses for the blocked solves, once after
 // the factorization.  Super-block K of a front (columns k0 = 256 K ..) is
 // made of up to four 64-column blocks with stored inverses D_s; its inverse
-// X follows by block forward substitution along the block sub-diagonals:
-//   X_ss = D_s,   X_st = -D_s sum_{u=t}^{s-1} L_su X_ut   (s > t),
-// 64 x 64 tile products in shared memory, 4 x 4 outputs per thread.
+// X follows by block forward substitution down each column block t:
+//   X_tt = D_t,   X_st = -D_s sum_{u=t}^{s-1} L_su X_ut   (s > t).
+// Columns of X are independent, so a CTA takes 32 of one block's: item
+// (front, K, 2 t + half).  Its X_ut stay in shared memory, and the next 64 x 64
+// operand is on its way in registers while the current one is multiplied:
+// doubles on DMMA (a warp 16 x 16 of the 64 x 32 product), floats as 4 x 2
+// FMAs a thread.  What bounds it is the chain of at most nine products (and on
+// trees of many super-blocks the reads of L).  One CTA for all of a
+// super-block, its scalar products bound by shared-memory reads, took 213 us
+// at 16^3, 267 us at KKT 24 and 804 us at 80^3 (FP64); this takes 33, 49 and
+// 612 us.
 // ---------------------------------------------------------------------------
 constexpr int ILD = kNB + 1;
+constexpr int kInvCols = kNB / 2;
 
 template <typename T>
-constexpr int inv256_smem() { return 3 * kNB * ILD * (int)sizeof(T); }
+constexpr int inv256_smem() { return (kNB * ILD + 5 * kInvCols * ILD) * (int)sizeof(T); }
 
-template <typename T>
-__device__ __forceinline__ void tile_in(T* dst, const T* src, int64_t ld, int rows, int cols) {
-    for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
-        const int r = e & (kNB - 1), c = e >> 6;
-        dst[r + c * ILD] = (r < rows && c < cols) ? src[r + (int64_t)c * ld] : T(0);
+// C(64 x 32) += A(64 x 64) B(64 x 32): A[r + k * ILD], B[k + c * ILD]; visit()
+// gives a thread's entries as (row, column, accumulator)
+struct InvAccD {
+    double c[2][2][2] = {};
+    __device__ __forceinline__ void mma(const double* A, const double* B) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int wr = (warp & 3) * 16, wc = (warp >> 2) * 16, fr = lane >> 2, fk = lane & 3;
+#pragma unroll 4
+        for (int k = 0; k < kNB; k += 4) {
+            double a[2], b[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) a[i] = A[(wr + 8 * i + fr) + (k + fk) * ILD];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) b[j] = B[(k + fk) + (wc + 8 * j + fr) * ILD];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) dmma(c[i][j][0], c[i][j][1], a[i], b[j]);
+        }
     }
-}
-
-template <typename T>
-__device__ __forceinline__ void tile_mma(T (&acc)[4][4], const T* A, const T* B) {
-    const int tr = (threadIdx.x >> 4) * 4, tc = (threadIdx.x & 15) * 4;
+    template <typename F>
+    __device__ __forceinline__ void visit(F&& fn) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int wr = (warp & 3) * 16, wc = (warp >> 2) * 16;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) fn(wr + 8 * i + (lane >> 2), wc + 8 * j + (lane & 3) * 2 + e, c[i][j][e]);
+    }
+};
+struct InvAccF {
+    float c[4][2] = {};
+    __device__ __forceinline__ void mma(const float* A, const float* B) {
+        const int tr = (threadIdx.x & 15) * 4, tc = (threadIdx.x >> 4) * 2;
 #pragma unroll 8
-    for (int k = 0; k < kNB; ++k) {
-        T a[4], b[4];
+        for (int k = 0; k < kNB; ++k) {
+            float a[4], b[2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = A[(tr + i) + k * ILD];
+            for (int i = 0; i < 4; ++i) a[i] = A[(tr + i) + k * ILD];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = B[k + (tc + j) * ILD];
+            for (int j = 0; j < 2; ++j) b[j] = B[k + (tc + j) * ILD];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) c[i][j] += a[i] * b[j];
+        }
+    }
+    template <typename F>
+    __device__ __forceinline__ void visit(F&& fn) {
+        const int tr = (threadIdx.x & 15) * 4, tc = (threadIdx.x >> 4) * 2;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * b[j];
+            for (int j = 0; j < 2; ++j) fn(tr + i, tc + j, c[i][j]);
     }
-}
+};
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_inv256(const Front* __restrict__ fronts, const Item* __restrict__ items,
                                                 const T* __restrict__ P, const T* __restrict__ inv,
                                                 T* __restrict__ inv2) {
     pdl_prologue();
+    using Acc2 = typename std::conditional<sizeof(T) == 8, InvAccD, InvAccF>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* As = reinterpret_cast<T*>(smem_raw);
-    T* Bs = As + kNB * ILD;
-    T* Cs = Bs + kNB * ILD;
+    T* Cs = As + kNB * ILD;               // the sum of a block row, as the next product's operand
+    T* Xs = Cs + kInvCols * ILD;          // X_ut, u = 0 .. 3
     const Item it = items[blockIdx.x];
     const Front f = fronts[it.front];
-    const int K = it.a, k0 = K * kSolveNB, wK = min(kSolveNB, f.nn - k0), ns = (wK + kNB - 1) / kNB;
-    const int ld2 = super_ld(wK), ld = f.ldp;
-    T* X = inv2 + f.i2off + (int64_t)K * kSolveNB * kSolveNB;
-    const T* Pj = P + f.poff;
-    const int tid = threadIdx.x;
-    for (int e = tid; e < ld2 * wK; e += blockDim.x) X[e] = T(0);
-    __syncthreads();
-    for (int s = 0; s < ns; ++s) {
+    const int K = it.a, t = it.b >> 1, cb = (it.b & 1) * kInvCols;
+    const int k0 = K * kSolveNB, wK = min(kSolveNB, f.nn - k0), ns = (wK + kNB - 1) / kNB;
+    const int ld2 = super_ld(wK), ld = f.ldp, tid = threadIdx.x;
+    const int nc = min(kInvCols, wK - t * kNB - cb);  // columns of the piece
+    T* X = inv2 + f.i2off + (int64_t)K * kSolveNB * kSolveNB + (int64_t)(t * kNB + cb) * ld2;
+    const T* Pk = P + f.poff + k0 + (int64_t)k0 * ld;
+    const T* Dk = inv + f.ioff + (int64_t)(k0 / kNB) * kNB * kNB;
+    // zeros above the block row t and in the padding rows
+    for (int e = tid; e < ld2 * nc; e += 256) {
+        const int r = e % ld2, c = e / ld2;
+        if (r < t * kNB || r >= wK) X[r + (int64_t)c * ld2] = T(0);
+    }
+    for (int e = tid; e < kNB * kInvCols; e += 256) {
+        const int r = e & (kNB - 1), c = e >> 6;
+        const T v = c < nc ? Dk[(int64_t)t * kNB * kNB + r + (cb + c) * kNB] : T(0);
+        Xs[t * kInvCols * ILD + r + c * ILD] = v;
+        if (c < nc && t * kNB + r < wK) X[t * kNB + r + (int64_t)c * ld2] = v;
+    }
+    // operands in the order they are needed: L_st .. L_s,s-1, D_s for each s
+    T v[16];
+    auto fetch = [&](int s, int u) {
         const int ws = min(kNB, wK - s * kNB);
-        const T* D = inv + f.ioff + (int64_t)(k0 / kNB + s) * kNB * kNB;
-        for (int e = tid; e < ws * ws; e += blockDim.x) {
-            const int r = e % ws, c = e / ws;
-            X[(s * kNB + r) + (int64_t)(s * kNB + c) * ld2] = D[r + c * kNB];
+        const T* src = u < s ? Pk + s * kNB + (int64_t)(u * kNB) * ld : Dk + (int64_t)s * kNB * kNB;
+        const int64_t l = u < s ? ld : kNB;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const int e = tid + 256 * q, r = e & (kNB - 1), c = e >> 6;
+            v[q] = r < ws ? src[r + c * l] : T(0);
+        }
+    };
+    if (t + 1 < ns) fetch(t + 1, t);
+    for (int s = t + 1; s < ns; ++s) {
+        const int ws = min(kNB, wK - s * kNB);
+        Acc2 sum, prod;
+        for (int u = t; u <= s; ++u) {
+            __syncthreads();  // As is free, Xs and Cs are whole
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const int e = tid + 256 * q;
+                As[(e & (kNB - 1)) + (e >> 6) * ILD] = v[q];
+            }
+            if (u < s) fetch(s, u + 1);
+            else if (s + 1 < ns) fetch(s + 1, t);
+            __syncthreads();
+            if (u < s) {
+                sum.mma(As, Xs + u * kInvCols * ILD);
+                if (u == s - 1) sum.visit([&](int r, int c, T x) { Cs[r + c * ILD] = x; });
+            } else {
+                prod.mma(As, Cs);
+                prod.visit([&](int r, int c, T x) {
+                    Xs[s * kInvCols * ILD + r + c * ILD] = -x;
+                    if (r < ws && c < nc) X[s * kNB + r + (int64_t)c * ld2] = -x;
+                });
+            }
         }
     }
-    __syncthreads();
-    const int tr = (tid >> 4) * 4, tc = (tid & 15) * 4;
-    for (int d = 1; d < ns; ++d)
-        for (int s = d; s < ns; ++s) {
-            const int t = s - d;
-            const int ws = min(kNB, wK - s * kNB), wt = min(kNB, wK - t * kNB);
-            T acc[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
-            for (int u = t; u < s; ++u) {  // T += L_su X_ut
-                tile_in(As, Pj + (k0 + s * kNB) + (int64_t)(k0 + u * kNB) * ld, ld, ws, kNB);
-                tile_in(Bs, X + u * kNB + (int64_t)(t * kNB) * ld2, ld2, kNB, wt);
-                __syncthreads();
-                tile_mma(acc, As, Bs);
-                __syncthreads();
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) Cs[(tr + i) + (tc + j) * ILD] = acc[i][j];
-            tile_in(As, inv + f.ioff + (int64_t)(k0 / kNB + s) * kNB * kNB, kNB, kNB, kNB);
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
-            tile_mma(acc, As, Cs);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (tr + i < ws && tc + j < wt)
-                        X[(s * kNB + tr + i) + (int64_t)(t * kNB + tc + j) * ld2] = -acc[i][j];
-            __syncthreads();  // X_st is read by the next distance
-        }
 }
 
 // ---------------------------------------------------------------------------

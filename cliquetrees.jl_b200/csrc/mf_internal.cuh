@@ -307,7 +307,7 @@ struct mf_handle {
     std::vector<int32_t> h_sepmap;          // reference sep rows -> execution panel rows
     std::vector<int64_t> h_resptr, h_sepptr, h_septgt, h_Dptr, h_Lptr;
     std::vector<mf::Level> levels;
-    mf::ItemList inv2_items;                // (front, super-block) of the super-block inverses
+    mf::ItemList inv2_items;                // (front, super-block, 32-column piece) of the super-block inverses
     std::vector<mf::Item> h_items;
 
     // device symbolic

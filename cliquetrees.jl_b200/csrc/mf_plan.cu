@@ -957,7 +957,9 @@ int build_plan(mf_handle* h, const int64_t* resptr, const int64_t* sepptr, const
     for (int64_t e = 0; e < (int64_t)h->h_fronts.size(); ++e) {
         const Front& f = h->h_fronts[(size_t)e];
         if (f.i2off < 0) continue;
-        for (int K = 0; K < (int)cdiv(f.nn, kSolveNB); ++K) push((int32_t)e, K, 0);
+        // 32-column pieces of every super-block, the longest chains (first block) first
+        for (int K = 0; K < (int)cdiv(f.nn, kSolveNB); ++K)
+            for (int c = 0; c < std::min(kSolveNB, f.nn - K * kSolveNB); c += kNB / 2) push((int32_t)e, K, c / (kNB / 2));
     }
     end(h->inv2_items);
     return 0;
