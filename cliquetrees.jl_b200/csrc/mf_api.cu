@@ -227,10 +227,12 @@ int mf_create(int64_t n, int64_t nfr, const int64_t* resptr, const int64_t* sepp
         h->tc_split = !(senv && senv[0] == '0');
         const char* cenv = getenv("MF_SOLVE_CHAIN");
         h->solve_chain = !cenv ? 2 : cenv[0] == '1' ? 1 : cenv[0] == '0' ? 0 : 2;
-        // the sub-panel chain launched for programmatic dependence measured
-        // no faster (80^3: 42.5 vs 42.2 ms; KKT: 232.6 vs 228.9 ms): opt-in
+        // setup and static loads beside the launch before: KKT 24 mixed 10.06
+        // -> 9.26 ms, 512^2 mixed 9.34 -> 8.61, 100^2 FP64 872 -> 791 us, 80^3
+        // within the noise.  (Launched early but waiting first, the sub-panel
+        // chain had gained nothing.)
         const char* ppenv = getenv("MF_PANEL_PDL");
-        h->panel_pdl = ppenv && ppenv[0] == '1';
+        h->panel_pdl = !(ppenv && ppenv[0] == '0');
         const char* fenv = getenv("MF_SIDE_FREE_SMS");
         if (fenv && atoi(fenv) >= 0) h->side_free_sms = atoi(fenv);
         const char* lenv = getenv("MF_LOOKAHEAD");

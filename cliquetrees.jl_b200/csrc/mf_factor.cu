@@ -379,12 +379,13 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // offsets are multiples of four entries), so they stream into shared memory
 // as 16-byte asynchronous copies, as many children at a time as `stage`
 // entries hold (at least the largest one), and the adds wait for one memory
-// trip per group instead of one per child.  Ends with a block barrier.
+// trip per group instead of one per child.  The panel (the assembled matrix)
+// and the children's records come before the wait for the level below.  Ends
+// with a block barrier.
 template <typename T>
 __device__ __forceinline__ void small_assemble(T* F, T* S, int stage, const Front& f,
                                                const Front* __restrict__ fronts, const int32_t* __restrict__ reltgt,
-                                               const int32_t* __restrict__ chdtgt, const T* __restrict__ P,
-                                               const T* __restrict__ M) {
+                                               const int32_t* __restrict__ chdtgt, const T* P, const T* M) {
     constexpr int V = 16 / (int)sizeof(T);
     const int nn = f.nn, nj = nn + f.na, ld = f.ldp;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
@@ -405,6 +406,8 @@ __device__ __forceinline__ void small_assemble(T* F, T* S, int stage, const Fron
             kid_sep0[q] = fc.sep0;
             kid_moff[q] = fc.moff;
         }
+        // the level below has written the children (and read what this front writes)
+        if (k0 == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
         __syncthreads();
         for (int q0 = 0; q0 < m;) {
             if (tid == 0) {  // the children of this group and where they land
@@ -442,6 +445,7 @@ __device__ __forceinline__ void small_assemble(T* F, T* S, int stage, const Fron
         }
     }
     if (nch == 0) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         cp_async_wait_all();
         __syncthreads();
     }
@@ -524,11 +528,10 @@ constexpr int kSmallRescue = 67;
 template <typename T, int LDLT, int TD, int R, bool REG>
 __global__ void __launch_bounds__(TD * TD) k_small(const Front* __restrict__ fronts, const Item* __restrict__ items,
                                                    int stage, const int32_t* __restrict__ reltgt,
-                                                   const int32_t* __restrict__ chdtgt, T* __restrict__ P,
-                                                   T* __restrict__ M, T* __restrict__ d,
+                                                   const int32_t* __restrict__ chdtgt, T* P, T* M, T* __restrict__ d,
                                                    const double* __restrict__ signs, long long* __restrict__ info,
                                                    int* __restrict__ rescued, Reg reg) {
-    pdl_prologue();
+    pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ ElimBufs<T, TD * R, false> s;
     __shared__ int flag;
@@ -775,11 +778,19 @@ __device__ __forceinline__ void ea_chunk(const int32_t* __restrict__ rel, const 
         if (r[u] >= 0) dst[r[u]] = o[u] + v[u];
 }
 
+//
+// A front may have hundreds of children that miss an item, and a small front's
+// item is a chain of dependent loads (child list, child record, relative
+// index, entry), so the lanes of a warp fetch the segments and records of 32
+// children at once -- and the first children's relative indices before the
+// kernel waits for the work below it -- and only children that reach the item
+// are visited.
 template <typename T, int PART>
 __global__ void __launch_bounds__(256) k_ea(const Front* __restrict__ fronts, const Item* __restrict__ items,
                                             const Item* __restrict__ all_items, const int32_t* __restrict__ reltgt,
-                                            T* __restrict__ P, T* __restrict__ M) {
-    pdl_prologue();
+                                            T* P, T* M) {
+    pdl_trigger();
+    constexpr unsigned kAll = 0xffffffffu;
     const Item it = items[blockIdx.x];
     const Front f = fronts[it.front];
     const int nn = f.nn, ld = f.ldp, lm = f.ldm;
@@ -789,30 +800,64 @@ __global__ void __launch_bounds__(256) k_ea(const Front* __restrict__ fronts, co
     T* Mj = M + f.moff;
     const Item* seg = all_items + it.pad;  // segment offsets index the whole item buffer
     const int nch = f.chd1 - f.chd0;
-    for (int s = 0; s < nch; ++s) {
-        const Item s1 = seg[2 * s], s2 = seg[2 * s + 1];
-        const int b0 = s1.a, b1 = s1.b, a0 = s2.front, a1 = s2.a;
-        if (b0 >= b1 || a1 <= a0) continue;
-        const Front fc = fronts[s1.front];
-        const int32_t* __restrict__ rel = reltgt + fc.sep0;
-        const T* Mc = M + fc.moff;
-        for (int b = b0; b < b1; ++b) {
-            const int col = __ldg(rel + b);
-            if (((col - c0) & 7) != warp) continue;  // the owner warp of this parent column
-            const T* mc = Mc + (int64_t)b * fc.ldm;
-            T* dst = PART == 0 ? Pj + (int64_t)col * ld : Mj + (int64_t)(col - nn) * lm - nn;
-            // full chunks of 4 x 32 rows, then one predicated chunk of at
-            // most 4 x 32 rows (a single row per lane when the rest is that
-            // short: many child columns are, and the predicated slots would
-            // cost instructions for nothing).  Eight chains per lane measured
-            // slower on long columns (more lines in flight than L1 keeps).
-            int a = max(a0, b) + lane;
-            for (; a + 96 < a1; a += 128) ea_chunk<T, 4, false>(rel, mc, dst, a, a1);
-            if (a + 32 < a1) ea_chunk<T, 4, true>(rel, mc, dst, a, a1);
-            else if (a < a1) dst[__ldg(rel + a)] += mc[a];
+    bool waited = false;
+    for (int s0 = 0; s0 < nch; s0 += 32) {
+        // lane q holds child s0 + q's segment and record
+        Item s1{}, s2{};
+        int sep0 = 0, ldm = 0;
+        int64_t moff = 0;
+        bool hit = false;
+        if (s0 + lane < nch) {
+            s1 = seg[2 * (s0 + lane)], s2 = seg[2 * (s0 + lane) + 1];
+            hit = s1.a < s1.b && s2.front < s2.a;
+            if (hit) {
+                const Front& fc = fronts[s1.front];
+                sep0 = fc.sep0, ldm = fc.ldm, moff = fc.moff;
+            }
         }
-        __syncwarp();
+        unsigned todo = __ballot_sync(kAll, hit);
+        int cn = -1;  // lane j: the parent column of the next child's column b0 + j
+        auto columns = [&](unsigned left) {
+            if (!left) return;
+            const int q = __ffs(left) - 1;
+            const int b0 = __shfl_sync(kAll, s1.a, q), b1 = __shfl_sync(kAll, s1.b, q), sp = __shfl_sync(kAll, sep0, q);
+            cn = b0 + lane < b1 ? __ldg(reltgt + sp + b0 + lane) : -1;
+        };
+        columns(todo);
+        if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+        waited = true;
+        while (todo) {
+            const int q = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int b0 = __shfl_sync(kAll, s1.a, q);
+            const int a0 = __shfl_sync(kAll, s2.front, q), a1 = __shfl_sync(kAll, s2.a, q);
+            const int32_t* __restrict__ rel = reltgt + __shfl_sync(kAll, sep0, q);
+            const T* Mc = M + __shfl_sync(kAll, moff, q);
+            const int lmc = __shfl_sync(kAll, ldm, q);
+            const int cq = cn;
+            columns(todo);
+            // the owner warp of a parent column takes it (at most kEAcols columns of the child fall in the item)
+            unsigned own = __ballot_sync(kAll, cq >= 0 && ((cq - c0) & 7) == warp);
+            while (own) {
+                const int j = __ffs(own) - 1;
+                own &= own - 1;
+                const int b = b0 + j, col = __shfl_sync(kAll, cq, j);
+                const T* mc = Mc + (int64_t)b * lmc;
+                T* dst = PART == 0 ? Pj + (int64_t)col * ld : Mj + (int64_t)(col - nn) * lm - nn;
+                // full chunks of 4 x 32 rows, then one predicated chunk of at
+                // most 4 x 32 rows (a single row per lane when the rest is that
+                // short: many child columns are, and the predicated slots would
+                // cost instructions for nothing).  Eight chains per lane measured
+                // slower on long columns (more lines in flight than L1 keeps).
+                int a = max(a0, b) + lane;
+                for (; a + 96 < a1; a += 128) ea_chunk<T, 4, false>(rel, mc, dst, a, a1);
+                if (a + 32 < a1) ea_chunk<T, 4, true>(rel, mc, dst, a, a1);
+                else if (a < a1) dst[__ldg(rel + a)] += mc[a];
+            }
+            __syncwarp();
+        }
     }
+    if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -887,10 +932,10 @@ __device__ __forceinline__ void diag_block_load(TC* A, TC* X, const T* Pj, int64
 // FP32.  A rejection in FP64 is reported through info.
 template <typename T, int LDLT, bool REG>
 __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                              int c0, T* __restrict__ P, T* __restrict__ inv,
+                                              int c0, T* P, T* __restrict__ inv,
                                               T* __restrict__ d, const double* __restrict__ signs,
                                               long long* __restrict__ info, int* __restrict__ rescued, Reg reg) {
-    pdl_prologue();
+    pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* A = reinterpret_cast<T*>(smem_raw);  // block, then its factor, A[r + c * LDA]
     T* X = A + kNB * LDA;                   // inverse, same layout
@@ -909,6 +954,7 @@ __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ front
     T* dst = inv + f.ioff + (int64_t)(c0 / kNB) * kNB * kNB;
     constexpr bool single = sizeof(T) == 4;
     if (tid == 0) { flag_s = 0; dmax_s = 0.0; }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     diag_block_load<T, T>(A, X, Pj, ld, c0, w);
     __syncthreads();
     // |a_kk| before the factorization and the block's largest (non-negative
@@ -1181,10 +1227,9 @@ __device__ __forceinline__ void g64_copy(double* dst, const double* src, int64_t
 template <int BM, int ROLE, int LDLT>
 __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64(const Front* __restrict__ fronts,
                                                                  const Item* __restrict__ items, int obs, int obw,
-                                                                 int c0, double* __restrict__ P,
-                                                                 double* __restrict__ M, const double* __restrict__ d,
+                                                                 int c0, double* P, double* M, const double* __restrict__ d,
                                                                  const double* __restrict__ inv) {
-    pdl_prologue();
+    pdl_trigger();
     constexpr int NT = g64_threads<BM>(), LA = BM + 4, LB = kTile + 4, STG = g64_stage<BM>();
     constexpr bool PAIR = BM == 128 && (ROLE == G_TRAIL || ROLE == G_SYRK);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1226,7 +1271,11 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
         Bm = inv + f.ioff + (int64_t)(c0 / kNB) * kNB * kNB - (int64_t)c0 * kNB;
         ldb = kNB, blim = kNB, tri = false;
     }
-    if (ra >= rhi || (tri && ra + BM <= rb)) return;  // past the rows, or wholly above the diagonal
+    // past the rows, or wholly above the diagonal (the wait is still taken: the
+    // next grid may rely on the one before this)
+    const bool none = ra >= rhi || (tri && ra + BM <= rb);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (none) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int WM = g64_wm<BM>(), MI = WM / 8;
     const int wr = (warp % (BM / WM)) * WM, wc = (warp / (BM / WM)) * 32;
@@ -1583,7 +1632,7 @@ int launch_panel32_to_dl(mf_handle* h, double* dD, double* dL) {
 template <int BM, int ROLE, int LDLT>
 static int gemm64_go(mf_handle* h, int64_t ctas, const Item* items, int obs, int obw, int c0,
                      const FactorBufs<double>& fb) {
-    const bool pdl = pdl_enabled() || (h->panel_pdl && (ROLE == G_LEFT || ROLE == G_TRSM));
+    const bool pdl = pdl_enabled() || (h->panel_pdl && ROLE != G_TRAIL);
     MF_CUDA(cudaFuncSetAttribute(k_gemm64<BM, ROLE, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, g64_smem<BM>()));
     launch_kx(pdl, k_gemm64<BM, ROLE, LDLT>, grid_for(ctas), g64_threads<BM>(), g64_smem<BM>(), h->stream, h->d_fronts,
               items, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
@@ -1634,7 +1683,7 @@ static int small_go(mf_handle* h, const ItemList& l, int mj, int stage, const Fa
     const size_t sm = std::max<size_t>(((size_t)stage + (size_t)lj * mj) * sizeof(T), sizeof(T) == 4 ? (size_t)rj * rj * 8 : 0);
     MF_CUDA(cudaFuncSetAttribute(k_small<T, LDLT, TD, R, REG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (kSmallStage + kSmallMax * kSmallMax) * (int)sizeof(T)));
-    launch_k(k_small<T, LDLT, TD, R, REG>, grid_for(l.cnt), TD * TD, sm, h->stream, h->d_fronts,
+    launch_kx(h->panel_pdl || pdl_enabled(), k_small<T, LDLT, TD, R, REG>, grid_for(l.cnt), TD * TD, sm, h->stream, h->d_fronts,
              h->d_items + l.off, stage, h->d_reltgt, h->d_chdtgt, fb.P, fb.M, fb.d, h->d_signs, h->d_info,
              h->d_rescued, reg);
     MF_CUDA(cudaGetLastError());
@@ -1709,7 +1758,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
         }
         if (lv.ea.cnt) {
             Timer t(h, K_EA);
-            launch_k(k_ea<T, 0>, grid_for(lv.ea.cnt), 256, 0, h->stream, h->d_fronts, items + lv.ea.off, items,
+            launch_kx(h->panel_pdl || pdl_enabled(), k_ea<T, 0>, grid_for(lv.ea.cnt), 256, 0, h->stream, h->d_fronts, items + lv.ea.off, items,
                                                                    h->d_reltgt, fb.P, fb.M);
             MF_CUDA(cudaGetLastError());
         }
@@ -1834,7 +1883,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
         }
         if (lv.ea_upd.cnt) {
             Timer t(h, K_EA);
-            launch_k(k_ea<T, 1>, grid_for(lv.ea_upd.cnt), 256, 0, h->stream, h->d_fronts, items + lv.ea_upd.off, items,
+            launch_kx(h->panel_pdl || pdl_enabled(), k_ea<T, 1>, grid_for(lv.ea_upd.cnt), 256, 0, h->stream, h->d_fronts, items + lv.ea_upd.off, items,
                                                                        h->d_reltgt, fb.P, fb.M);
             MF_CUDA(cudaGetLastError());
         }

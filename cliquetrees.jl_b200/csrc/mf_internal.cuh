@@ -351,8 +351,9 @@ struct mf_handle {
     int solve_chain = 2;           // k_s_chain launches: 1 every level (MF_SOLVE_CHAIN=1), 0 none (=0),
                                    // 2 the levels of at least kChainMinSteps steps (default)
     bool tiny_solve = true;        // k_s_tiny_* for the fronts with nj <= kTinyNJ (MF_TINY_SOLVE=0: k_s_small_*)
-    bool panel_pdl = false;        // the factorization's sub-panel chain (left-looking, diagonal block, TRSM)
-                                   // launched for programmatic dependence (MF_PANEL_PDL=1)
+    bool panel_pdl = true;         // the factorization's short launches (small fronts, extend-add, left-looking,
+                                   // diagonal block, TRSM, SYRK) launched for programmatic dependence: setup
+                                   // and static loads beside the launch before (MF_PANEL_PDL=0: off)
     cudaStream_t side = nullptr;   // the factorization's look-ahead stream (trailing updates beside the next
                                    // outer block's sub-panels), forked from and joined into `stream`
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

@@ -323,12 +323,12 @@ __device__ __forceinline__ TileGeom tile_geom(const Front* __restrict__ fronts, 
 template <int ROLE, int LDLT, bool SPLIT>
 __global__ void __launch_bounds__(tc::NT, 1) k_gemm_tc(const Front* __restrict__ fronts,
                                                        const Item* __restrict__ items, int64_t ntiles, int obs, int obw, int c0,
-                                                       float* __restrict__ P, float* __restrict__ M,
+                                                       float* P, float* M,
                                                        const float* __restrict__ d,
                                                        const CUtensorMap* __restrict__ maps,
                                                        const CUtensorMap* __restrict__ inv_map,
                                                        const float* __restrict__ split, int* __restrict__ err) {
-    pdl_prologue();
+    pdl_trigger();
     using namespace tc;
     constexpr int TN = TcTileN<ROLE>::value;
     using C_ = Cfg<TN>;
@@ -369,6 +369,8 @@ __global__ void __launch_bounds__(tc::NT, 1) k_gemm_tc(const Front* __restrict__
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    // barriers and TMEM are set up beside the tail of the grid before this one
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     auto fail = [&](int code) {
         *abort = 1;
         atomicExch(err, code);
@@ -581,7 +583,7 @@ static int launch_one(mf_handle* h, const ItemList& l, int obs, int obw, int c0,
     if (!l.cnt) return 0;
     constexpr int smem = tc::Cfg<TcTileN<ROLE>::value>::SMEM_BYTES;
     const int64_t grid = std::min<int64_t>(l.cnt, h->grid_cap > 0 ? h->grid_cap : h->num_sms > 0 ? h->num_sms : 148);
-    launch_kx(pdl_enabled() || (h->panel_pdl && (ROLE == 0 || ROLE == 3)), k_gemm_tc<ROLE, LDLT, false>,
+    launch_kx(pdl_enabled() || (h->panel_pdl && (ROLE == TC_LEFT || ROLE == TC_TRSM)), k_gemm_tc<ROLE, LDLT, false>,
               (unsigned)grid, tc::NT, smem, h->stream, 
         h->d_fronts, h->d_items + l.off, l.cnt, obs, obw, c0, fb.P, fb.M, fb.d,
         reinterpret_cast<const CUtensorMap*>(h->d_tmaps), reinterpret_cast<const CUtensorMap*>(h->d_tmap_inv),
@@ -665,7 +667,7 @@ static int launch_split(mf_handle* h, const ItemList& l, const ItemList& units, 
     }
     constexpr int smem = tc::SplitCfg<TcTileN<ROLE>::value>::SMEM_BYTES;
     const int64_t grid = std::min<int64_t>(l.cnt, h->grid_cap > 0 ? h->grid_cap : h->num_sms > 0 ? h->num_sms : 148);
-    launch_k(k_gemm_tc<ROLE, LDLT, true>, (unsigned)grid, tc::NT, smem, h->stream, 
+    launch_kx(pdl_enabled() || (h->panel_pdl && units.cnt > 0), k_gemm_tc<ROLE, LDLT, true>, (unsigned)grid, tc::NT, smem, h->stream, 
         h->d_fronts, h->d_items + l.off, l.cnt, obs, obw, c0, fb.P, fb.M, fb.d,
         reinterpret_cast<const CUtensorMap*>(h->d_tmaps), reinterpret_cast<const CUtensorMap*>(h->d_tmap_inv),
         h->f32.split, h->d_err);
