@@ -435,9 +435,26 @@ __device__ __forceinline__ void small_assemble(T* F, T* S, int stage, const Fron
                 const int ma = kid_na[q], lm = kid_lm[q];
                 const int32_t* rel = kid_rel + q * kSmallMax;
                 const T* Mc = S + kid_at[q];
-                for (int b = warp; b < ma; b += nw) {
-                    T* col = F + rel[b] * ld;
-                    for (int r = b + lane; r < ma; r += 32) col[rel[r]] += Mc[r + b * lm];
+                // a child's entries land on distinct entries of F, so a lane
+                // reads four columns' worth before it writes the first
+                for (int b0 = warp; b0 < ma; b0 += 4 * nw) {
+                    int col[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) col[u] = b0 + u * nw < ma ? rel[b0 + u * nw] * ld : 0;
+                    for (int r = (b0 & ~31) + lane; r < ma; r += 32) {
+                        const int rr = rel[r];
+                        T v[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int b = b0 + u * nw;
+                            v[u] = (b <= r && b < ma) ? F[col[u] + rr] + Mc[r + b * lm] : T(0);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int b = b0 + u * nw;
+                            if (b <= r && b < ma) F[col[u] + rr] = v[u];
+                        }
+                    }
                 }
                 __syncthreads();
             }
