@@ -42,28 +42,6 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v) {
     atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
-// y = A x for nrhs columns (ld n); values read through the stored-value map
-__global__ void k_spmv(const int64_t* __restrict__ ptr, const int32_t* __restrict__ col,
-                       const int64_t* __restrict__ src, const double* __restrict__ nz, const double* __restrict__ x,
-                       double* __restrict__ y, int64_t n, int nrhs) {
-    pdl_prologue();
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double acc[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) acc[r] = 0.0;
-    for (int64_t p = ptr[i]; p < ptr[i + 1]; ++p) {
-        const double a = nz[src[p]];
-        const int64_t c = col[p];
-#pragma unroll
-        for (int r = 0; r < 16; ++r)
-            if (r < nrhs) acc[r] += a * x[c + r * n];
-    }
-#pragma unroll
-    for (int r = 0; r < 16; ++r)
-        if (r < nrhs) y[i + r * n] = acc[r];
-}
-
 // t = b - A x for row i (all columns) with the stored-value map; the
 // products are added in the row's stored order
 template <int NR>
@@ -82,6 +60,25 @@ __device__ __forceinline__ void resid_row(const int64_t* __restrict__ ptr, const
         for (int r = 0; r < NR; ++r)
             if (r < nrhs) acc[r] += a * x[c + r * n];
     }
+}
+
+// y = A x for nrhs columns (ld n).  NR, the right-hand sides the row's sums
+// are held for, follows nrhs: with sixteen sums whatever nrhs was, a row's
+// entries came one memory trip at a time (batch of 512 2D systems, four
+// right-hand sides: 57 us a product; 39 us with NR = 4, four entries in flight)
+template <int NR>
+__global__ void __launch_bounds__(256) k_spmv(const int64_t* __restrict__ ptr, const int32_t* __restrict__ col,
+                                              const int64_t* __restrict__ src, const double* __restrict__ nz,
+                                              const double* __restrict__ x, double* __restrict__ y, int64_t n,
+                                              int nrhs) {
+    pdl_prologue();
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double acc[NR];
+    resid_row<NR>(ptr, col, src, nz, x, i, n, nrhs, acc);
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+        if (r < nrhs) y[i + r * n] = acc[r];
 }
 
 // t = b - A x and the maxima needed by the backward error:
@@ -175,27 +172,48 @@ __global__ void k_seg_zero(double* __restrict__ segred, int64_t nseg) {
     if (i < nseg * 48) segred[(i / 48) * kSegRed + i % 48] = 0.0;
 }
 
-// per chunk and column: sum of u .* v over the chunk's rows into
-// chunkred[c * kChunkRed + kSegRed + r]
-__global__ void k_dot_chunk(const double* __restrict__ u, const double* __restrict__ v,
-                            const int64_t* __restrict__ chunkrow, double* __restrict__ chunkred, int64_t n,
-                            int nrhs) {
-    pdl_prologue();
-    __shared__ double sh[256];
-    const int64_t c = blockIdx.x;
-    const int64_t r0 = chunkrow[c], r1 = chunkrow[c + 1];
-    for (int r = 0; r < nrhs; ++r) {
-        double s = 0.0;
-        for (int64_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) s += u[i + r * n] * v[i + r * n];
-        sh[threadIdx.x] = s;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) chunkred[c * kChunkRed + kSegRed + r] = sh[0];
+// sums of u .* v over the rows r0 + thread, step, ... < r1 of the block, one
+// per column, added over the 256 threads in the fixed order of halving
+// strides; out[r] gets column r.  All columns go together: one pass over the
+// rows and four barriers (column by column, nine barriers each, a batch's dot
+// took 15.6 us for four columns; 11.8 us this way)
+template <int NR>
+__device__ __forceinline__ void block_dots(const double* __restrict__ u, const double* __restrict__ v, int64_t r0,
+                                           int64_t r1, int64_t step, int64_t n, int nrhs, double* __restrict__ out) {
+    __shared__ double sh[NR][256];
+    const int tid = threadIdx.x, lane = tid & 31;
+    double s[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) s[r] = 0.0;
+    for (int64_t i = r0 + tid; i < r1; i += step)
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+            if (r < nrhs) s[r] += u[i + r * n] * v[i + r * n];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) sh[r][tid] = s[r];
+    __syncthreads();
+    for (int o = 128; o >= 32; o >>= 1) {
+        if (tid < o)
+#pragma unroll
+            for (int r = 0; r < NR; ++r) sh[r][tid] += sh[r][tid + o];
         __syncthreads();
     }
+    for (int r = tid >> 5; r < nrhs; r += 8) {
+        double x = sh[r][lane];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) out[r] = x;
+    }
+}
+
+// per chunk and column: sum of u .* v over the chunk's rows into
+// chunkred[c * kChunkRed + kSegRed + r]
+template <int NR>
+__global__ void __launch_bounds__(256) k_dot_chunk(const double* __restrict__ u, const double* __restrict__ v,
+                                                   const int64_t* __restrict__ chunkrow, double* __restrict__ chunkred,
+                                                   int64_t n, int nrhs) {
+    pdl_prologue();
+    const int64_t c = blockIdx.x;
+    block_dots<NR>(u, v, chunkrow[c], chunkrow[c + 1], 256, n, nrhs, chunkred + c * kChunkRed + kSegRed);
 }
 
 // out[s * 80 + r] = sum over the chunks of segment s (fixed order)
@@ -261,35 +279,27 @@ __global__ void k_anorm(const int64_t* __restrict__ ptr, const int64_t* __restri
 }
 
 // per-column partial dot products: part[blk * 16 + r]
-__global__ void k_dot_part(const double* __restrict__ u, const double* __restrict__ v, double* __restrict__ part,
-                           int64_t n, int nrhs) {
+template <int NR>
+__global__ void __launch_bounds__(256) k_dot_part(const double* __restrict__ u, const double* __restrict__ v,
+                                                  double* __restrict__ part, int64_t n, int nrhs) {
     pdl_prologue();
-    __shared__ double sh[256];
-    for (int r = 0; r < nrhs; ++r) {
-        double s = 0.0;
-        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-            s += u[i + r * n] * v[i + r * n];
-        sh[threadIdx.x] = s;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) part[blockIdx.x * 16 + r] = sh[0];
-        __syncthreads();
-    }
+    block_dots<NR>(u, v, blockIdx.x * (int64_t)blockDim.x, n, (int64_t)gridDim.x * blockDim.x, n, nrhs,
+                   part + blockIdx.x * 16);
 }
 
 // out[r] = sum over blocks (fixed order)
 // one warp per right-hand side: lane l adds blocks l, l + 32, ... in order,
 // then a fixed shuffle tree (deterministic, and the loads of a lane are
 // independent instead of one dependent chain over all blocks)
-__global__ void k_dot_final(const double* __restrict__ part, double* __restrict__ out, int nblocks, int nrhs) {
+__global__ void k_dot_final(const double* __restrict__ part, double* __restrict__ out, int nrhs) {
     pdl_prologue();
     const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (r >= nrhs) return;
-    double s = 0.0;
-    for (int b = lane; b < nblocks; b += 32) s += part[b * 16 + r];
+    double x[(kRedBlocks + 31) / 32], s = 0.0;  // all in flight: one trip to L2, not nineteen
+#pragma unroll
+    for (int i = 0; i < (kRedBlocks + 31) / 32; ++i) x[i] = lane + 32 * i < kRedBlocks ? part[(lane + 32 * i) * 16 + r] : 0.0;
+#pragma unroll
+    for (int i = 0; i < (kRedBlocks + 31) / 32; ++i) s += x[i];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) out[r] = s;
 }
@@ -400,26 +410,16 @@ __global__ void k_from32(double* __restrict__ z, const float* __restrict__ c, co
 constexpr int kGmresM = 24;  // restart length
 
 // part[(blk * J + i) * 16 + r] = this block's share of <V_i(:, r), w(:, r)>
-__global__ void k_mdot_part(const double* __restrict__ V, int64_t vs, int J, const double* __restrict__ w,
-                            double* __restrict__ part, int64_t n, int nrhs) {
+template <int NR>
+__global__ void __launch_bounds__(256) k_mdot_part(const double* __restrict__ V, int64_t vs, int J,
+                                                   const double* __restrict__ w, double* __restrict__ part, int64_t n,
+                                                   int nrhs) {
     pdl_prologue();
-    __shared__ double sh[256];
-    for (int i = 0; i < J; ++i)
-        for (int r = 0; r < nrhs; ++r) {
-            const double* v = V + i * vs + (int64_t)r * n;
-            const double* ww = w + (int64_t)r * n;
-            double s = 0.0;
-            for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-                s += v[k] * ww[k];
-            sh[threadIdx.x] = s;
-            __syncthreads();
-            for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-                if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-                __syncthreads();
-            }
-            if (threadIdx.x == 0) part[((int64_t)blockIdx.x * J + i) * 16 + r] = sh[0];
-            __syncthreads();
-        }
+    for (int i = 0; i < J; ++i) {
+        if (i) __syncthreads();  // the sums before have been read
+        block_dots<NR>(V + i * vs, w, blockIdx.x * (int64_t)blockDim.x, n, (int64_t)gridDim.x * blockDim.x, n, nrhs,
+                       part + ((int64_t)blockIdx.x * J + i) * 16);
+    }
 }
 
 // out[i * 16 + r] = sum over blocks (fixed order)
@@ -462,27 +462,16 @@ __global__ void k_colscale(double* __restrict__ dst, const double* __restrict__ 
 // Segmented forms of the GMRES kernels: a right-hand side of every segment
 // has its own Krylov space, so coefficients are indexed (i, segment, column)
 // as c[(i * G + s) * 16 + r] with G segments.
-__global__ void k_mdot_chunk(const double* __restrict__ V, int64_t vs, int J, const double* __restrict__ w,
-                             const int64_t* __restrict__ chunkrow, double* __restrict__ part, int64_t n, int nrhs) {
+template <int NR>
+__global__ void __launch_bounds__(256) k_mdot_chunk(const double* __restrict__ V, int64_t vs, int J,
+                                                    const double* __restrict__ w, const int64_t* __restrict__ chunkrow,
+                                                    double* __restrict__ part, int64_t n, int nrhs) {
     pdl_prologue();
-    __shared__ double sh[256];
     const int64_t c = blockIdx.x;
-    const int64_t r0 = chunkrow[c], r1 = chunkrow[c + 1];
-    for (int i = 0; i < J; ++i)
-        for (int r = 0; r < nrhs; ++r) {
-            const double* v = V + i * vs + (int64_t)r * n;
-            const double* ww = w + (int64_t)r * n;
-            double sum = 0.0;
-            for (int64_t k = r0 + threadIdx.x; k < r1; k += blockDim.x) sum += v[k] * ww[k];
-            sh[threadIdx.x] = sum;
-            __syncthreads();
-            for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-                if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-                __syncthreads();
-            }
-            if (threadIdx.x == 0) part[(c * J + i) * 16 + r] = sh[0];
-            __syncthreads();
-        }
+    for (int i = 0; i < J; ++i) {
+        if (i) __syncthreads();  // the sums before have been read
+        block_dots<NR>(V + i * vs, w, chunkrow[c], chunkrow[c + 1], 256, n, nrhs, part + (c * J + i) * 16);
+    }
 }
 __global__ void k_mdot_seg(const double* __restrict__ part, const int64_t* __restrict__ segchunk,
                            double* __restrict__ out, int64_t G, int J, int nrhs) {
@@ -571,9 +560,13 @@ static int apply_prec(mf_handle* h, const double* r, double* z, int nrhs) {
 
 static int dot(mf_handle* h, const double* u, const double* v, double* out, int nrhs) {
     double* part = h->d_red + kRedPart;
-    launch_k(k_dot_part, kRedBlocks, 256, 0, h->stream, u, v, part, h->n, nrhs);
+#define MF_DOT(NRV) launch_k(k_dot_part<NRV>, kRedBlocks, 256, 0, h->stream, u, v, part, h->n, nrhs)
+    if (nrhs <= 1) MF_DOT(1);
+    else if (nrhs <= 4) MF_DOT(4);
+    else MF_DOT(16);
+#undef MF_DOT
     MF_CUDA(cudaGetLastError());
-    launch_k(k_dot_final, 1, 32 * 16, 0, h->stream, part, out, kRedBlocks, nrhs);
+    launch_k(k_dot_final, 1, 32 * 16, 0, h->stream, part, out, nrhs);
     MF_CUDA(cudaGetLastError());
     return 0;
 }
@@ -581,11 +574,30 @@ static int dot(mf_handle* h, const double* u, const double* v, double* out, int 
 // per-segment dot products into h->d_segsc[s * 80 + off + r]
 static int dot_seg(mf_handle* h, const double* u, const double* v, int off, int nrhs) {
     if (h->nchunk > 0) {
-        launch_k(k_dot_chunk, (unsigned)h->nchunk, 256, 0, h->stream, u, v, h->d_chunkrow, h->d_chunkred, h->n, nrhs);
+#define MF_DOT(NRV) \
+    launch_k(k_dot_chunk<NRV>, (unsigned)h->nchunk, 256, 0, h->stream, u, v, h->d_chunkrow, h->d_chunkred, h->n, nrhs)
+        if (nrhs <= 1) MF_DOT(1);
+        else if (nrhs <= 4) MF_DOT(4);
+        else MF_DOT(16);
+#undef MF_DOT
         MF_CUDA(cudaGetLastError());
     }
     launch_k(k_dot_seg, (unsigned)((h->nseg * 16 + 255) / 256), 256, 0, h->stream, h->d_chunkred, h->d_segchunk,
                                                                              h->d_segsc + off, h->nseg, nrhs);
+    MF_CUDA(cudaGetLastError());
+    return 0;
+}
+
+static int spmv(mf_handle* h, const double* x, double* y, int nrhs) {
+#define MF_SPMV(NRV)                                                                                            \
+    launch_k(k_spmv<NRV>, row_blocks(h->n), 256, 0, h->stream, h->d_csrptr, h->d_csrcol, h->d_csrsrc, h->cur_nz, x, \
+             y, h->n, nrhs)
+    if (nrhs <= 1) MF_SPMV(1);
+    else if (nrhs <= 2) MF_SPMV(2);
+    else if (nrhs <= 4) MF_SPMV(4);
+    else if (nrhs <= 8) MF_SPMV(8);
+    else MF_SPMV(16);
+#undef MF_SPMV
     MF_CUDA(cudaGetLastError());
     return 0;
 }
@@ -684,13 +696,22 @@ static int gmres(mf_handle* h, const double* b, double* x, int nrhs, double tol,
     auto mdot = [&](const double* Vb, int J, const double* w, double* out_host) -> int {
         if (seg) {
             if (h->nchunk > 0) {
-                launch_k(k_mdot_chunk, (unsigned)h->nchunk, 256, 0, h->stream, Vb, vs, J, w, h->d_chunkrow, part, n, nrhs);
+#define MF_DOT(NRV) \
+    launch_k(k_mdot_chunk<NRV>, (unsigned)h->nchunk, 256, 0, h->stream, Vb, vs, J, w, h->d_chunkrow, part, n, nrhs)
+                if (nrhs <= 1) MF_DOT(1);
+                else if (nrhs <= 4) MF_DOT(4);
+                else MF_DOT(16);
+#undef MF_DOT
                 MF_CUDA(cudaGetLastError());
             }
             launch_k(k_mdot_seg, (unsigned)((J * Q + 255) / 256), 256, 0, h->stream, part, h->d_segchunk, coef, G, J,
                                                                                 nrhs);
         } else {
-            launch_k(k_mdot_part, nblk, 256, 0, h->stream, Vb, vs, J, w, part, n, nrhs);
+#define MF_DOT(NRV) launch_k(k_mdot_part<NRV>, nblk, 256, 0, h->stream, Vb, vs, J, w, part, n, nrhs)
+            if (nrhs <= 1) MF_DOT(1);
+            else if (nrhs <= 4) MF_DOT(4);
+            else MF_DOT(16);
+#undef MF_DOT
             MF_CUDA(cudaGetLastError());
             launch_k(k_mdot_final, (unsigned)((J * 16 + 7) / 8), 256, 0, h->stream, part, coef, nblk, J, nrhs);
         }
@@ -759,9 +780,7 @@ static int gmres(mf_handle* h, const double* b, double* x, int nrhs, double tol,
             ++used;
             {
                 Timer tm(h, K_SPMV);
-                launch_k(k_spmv, row_blocks(n), 256, 0, h->stream, h->d_csrptr, h->d_csrcol, h->d_csrsrc, h->cur_nz, Zj, w,
-                                                              n, nrhs);
-                MF_CUDA(cudaGetLastError());
+                if ((rc = spmv(h, Zj, w, nrhs))) return rc;
             }
             // classical Gram-Schmidt, twice
             for (int pass = 0; pass < 2; ++pass) {
@@ -884,9 +903,7 @@ int refine(mf_handle* h, const double* b, double* x, int nrhs, double tol, int m
         for (it = 1; it <= maxit; ++it) {
             {
                 Timer tm(h, K_SPMV);
-                launch_k(k_spmv, row_blocks(n), 256, 0, h->stream, h->d_csrptr, h->d_csrcol, h->d_csrsrc, h->cur_nz, Pv, Q,
-                                                              n, nrhs);
-                MF_CUDA(cudaGetLastError());
+                if ((rc = spmv(h, Pv, Q, nrhs))) return rc;
             }
             if ((rc = dotv(Pv, Q, 16))) return rc;  // pq
             if ((rc = scalars(0))) return rc;
