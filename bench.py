@@ -257,14 +257,14 @@ def exec_sizes(lib, h):
 
 # kernel families of the profiled classes (csrc/)
 CLASS_KERNELS = {
-    "syrk": "k_gemm_tc<2> (FP32: tcgen05 TF32) / k_gemm<double,2> (FP64: DMMA)",
-    "update": "k_gemm_tc<1> / k_gemm<T,1> trailing update",
-    "left": "k_gemm_tc<0> / k_gemm<T,0> left-looking update",
-    "panel": "k_gemm_tc<3> / k_gemm<T,3> panel TRSM (product with the block inverse)",
+    "syrk": "k_gemm_tc<2> (FP32: tcgen05 TF32) / k_gemm64<BM,2> (FP64: DMMA)",
+    "update": "k_gemm_tc<1> / k_gemm<float,1> / k_gemm64<BM,1> trailing update",
+    "left": "k_gemm_tc<0> / k_gemm<float,0> / k_gemm64<BM,0> left-looking update",
+    "panel": "k_gemm_tc<3> / k_gemm<float,3> / k_gemm64<BM,3> panel TRSM (product with the block inverse)",
     "diag": "k_diag 64x64 diagonal factor + inverse",
     "small": "k_small fused small fronts",
     "extend_add": "k_ea extend-add",
-    "solve_small": "k_s_small_fwd / k_s_small_bwd",
+    "solve_small": "k_s_cta_fwd/bwd, k_s_small_fwd/bwd, k_s_tiny_fwd/bwd",
     "solve_fwd": "k_s_sdiag + k_s_ftile forward steps",
     "solve_bwd": "k_s_sdiag + k_s_btile backward steps",
     "solve_bwd_l": "k_s_bwd_l + k_s_bwd_red backward L21^T x[sep]",

@@ -928,7 +928,7 @@ __device__ void diag_block_store(const TC* A, const TC* X, const TC* pivs, int w
     }
 }
 
-template <typename TC, typename T>
+template <typename TC, typename T, bool ZERO>
 __device__ __forceinline__ void diag_block_load(TC* A, TC* X, const T* Pj, int64_t ld, int c0, int w) {
     const int tid = threadIdx.x;
 #pragma unroll
@@ -937,22 +937,117 @@ __device__ __forceinline__ void diag_block_load(TC* A, TC* X, const T* Pj, int64
         TC v = (r == c) ? TC(1) : TC(0);
         if (r >= c && r < w && c < w) v = (TC)Pj[(c0 + r) + (int64_t)(c0 + c) * ld];
         A[r + c * LDA] = v;
-        X[r + c * LDA] = TC(0);
+        if (ZERO) X[r + c * LDA] = TC(0);
     }
 }
 
-// Diagonal block kernel.  Single precision: when the FP32 factorization
-// rejects a pivot, or a pivot lost more than five digits against its
-// diagonal entry or grew beyond 1e7 times the block's largest diagonal entry,
-// the block is loaded again and factored and inverted in FP64 (the dynamic
-// shared memory is sized for that), and the FP64 result is stored rounded to
-// FP32.  A rejection in FP64 is reported through info.
-template <typename T, int LDLT, bool REG>
+// FP64: the block's left-looking update from the outer block's columns
+// [k0, c0), sum_k (L_rk d_k) L_ck over its lower triangle, in chunks of 64
+// columns staged as stage[k * DLD + row] while the next chunk is on its way in
+// registers; on DMMA, the triangle's 36 8 x 8 tiles nine a pair of warps
+// (w, w + 4) that share a scheduler (tile row 7 - s and tile row s).
+constexpr int DLD = kNB + 4;
+struct DiagAccD {
+    double c[5][2] = {};
+    __device__ __forceinline__ static void tile(int t, int& r, int& col, bool& ok) {
+        const int warp = threadIdx.x >> 5, s = warp & 3;
+        if (warp < 4) { r = 7 - s; col = t; ok = true; }
+        else if (t < 3 - s) { r = 7 - s; col = 5 + t; ok = true; }
+        else { r = s; col = t - (3 - s); ok = col <= s; }
+    }
+    template <int LDLT>
+    __device__ __forceinline__ void mma(const double* S, const double* dsc) {
+        const int lane = threadIdx.x & 31, fr = lane >> 2, fk = lane & 3;
+        const int s = (threadIdx.x >> 5) & 3, r0 = 8 * (7 - s) + fr, r1 = 8 * s + fr;
+        int co[5];
+        bool first[5], ok[5];  // all uniform in a warp
+#pragma unroll
+        for (int t = 0; t < 5; ++t) {
+            int r, col;
+            tile(t, r, col, ok[t]);
+            first[t] = r == 7 - s;
+            co[t] = ok[t] ? 8 * col + fr : 0;
+        }
+#pragma unroll 4
+        for (int k = 0; k < kNB; k += 4) {
+            const double* Sk = S + (k + fk) * DLD;
+            double a0 = Sk[r0], a1 = Sk[r1];
+            if (LDLT) a0 *= dsc[k + fk], a1 *= dsc[k + fk];
+#pragma unroll
+            for (int t = 0; t < 5; ++t)
+                if (ok[t]) dmma(c[t][0], c[t][1], first[t] ? a0 : a1, Sk[co[t]]);
+        }
+    }
+    template <typename F>
+    __device__ __forceinline__ void visit(F&& fn) {
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int t = 0; t < 5; ++t) {
+            int r, col;
+            bool ok;
+            tile(t, r, col, ok);
+            if (ok)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) fn(8 * r + (lane >> 2), 8 * col + (lane & 3) * 2 + e, c[t][e]);
+        }
+    }
+};
+template <int LDLT>
+__device__ __forceinline__ void diag_update(double* A, double* X, double* dsc, const double* Pj, const double* dj,
+                                            int64_t ld, int k0, int c0, int w) {
+    constexpr int PER = kNB * kNB / 256;
+    const int tid = threadIdx.x, r = tid & (kNB - 1), kc = tid >> 6;
+    double* stage = X;  // X's place and 1.5 KB of the elimination's buffers after it
+    DiagAccD acc;
+    double v[PER], dv = 0.0;
+    auto fetch = [&](int k) {
+#pragma unroll
+        for (int u = 0; u < PER; ++u) v[u] = r < w ? Pj[(c0 + r) + (int64_t)(k + kc + 4 * u) * ld] : 0.0;
+        if (LDLT && tid < kNB) dv = dj[k + tid];
+    };
+    fetch(k0);
+    diag_block_load<double, double, false>(A, X, Pj, ld, c0, w);
+    for (int k = k0; k < c0; k += kNB) {
+#pragma unroll
+        for (int u = 0; u < PER; ++u) stage[(kc + 4 * u) * DLD + r] = v[u];
+        if (LDLT && tid < kNB) dsc[tid] = dv;
+        __syncthreads();
+        if (k + kNB < c0) fetch(k + kNB);
+        acc.mma<LDLT>(stage, dsc);
+        __syncthreads();
+    }
+    for (int e = tid; e < kNB * LDA; e += 256) X[e] = 0.0;
+    acc.visit([&](int row, int col, double x) {
+        if (row >= col && row < w) A[row + col * LDA] -= x;  // (col <= row < w)
+    });
+}
+static_assert(kNB * DLD <= kNB * LDA + 4 * kNB, "the stage ends inside the elimination's buffers");
+
+// Diagonal block kernel.  UPDATE (FP64, sub-panels after an outer block's
+// first): applies the block's left-looking update before it factors and
+// inverts it.  The rows below get theirs from the LEFT launch that follows,
+// which runs beside this one: a sub-panel's chain is the longer of the two and
+// the TRSM, not their sum.  For that this kernel lets the next grid go only
+// after its own wait, when all that both read is complete, and LEFT waits for
+// this kernel at its end.  KKT 24 10.78 -> 10.30 ms (a sub-panel's update and
+// block 25 -> 23 us, and its rows' update off the chain), 80^3 81.1 -> 79.3,
+// 16^3 1.182 -> 1.168 ms.
+// Not in single precision: on the chain the update costs the 64 x 64 x K
+// products on one SM, about what the tensor-core launch took (KKT 24 mixed
+// 9.08 -> 9.04 ms, 80^3 mixed 32.65 -> 32.80, 512^2 8.56 -> 8.55).
+//
+// Single precision: when the FP32 factorization rejects a pivot, or a pivot
+// lost more than five digits against its diagonal entry or grew beyond 1e7
+// times the block's largest diagonal entry, the block is loaded again and
+// factored and inverted in FP64 (the dynamic shared memory is sized for that),
+// and the FP64 result is stored rounded to FP32.  A rejection in FP64 is
+// reported through info.
+template <typename T, int LDLT, bool REG, bool UPDATE>
 __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                              int c0, T* P, T* __restrict__ inv,
+                                              int obs, int c0, T* P, T* __restrict__ inv,
                                               T* __restrict__ d, const double* __restrict__ signs,
                                               long long* __restrict__ info, int* __restrict__ rescued, Reg reg) {
-    pdl_trigger();
+    if (!UPDATE) pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* A = reinterpret_cast<T*>(smem_raw);  // block, then its factor, A[r + c * LDA]
     T* X = A + kNB * LDA;                   // inverse, same layout
@@ -972,7 +1067,14 @@ __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ front
     constexpr bool single = sizeof(T) == 4;
     if (tid == 0) { flag_s = 0; dmax_s = 0.0; }
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    diag_block_load<T, T>(A, X, Pj, ld, c0, w);
+    if constexpr (UPDATE) {
+        static_assert(!single, "FP64 only");
+        pdl_trigger();
+        __shared__ double dsc[LDLT ? kNB : 1];
+        diag_update<LDLT>(A, X, dsc, Pj, d + f.col0, ld, obs, c0, w);
+    } else {
+        diag_block_load<T, T, true>(A, X, Pj, ld, c0, w);
+    }
     __syncthreads();
     // |a_kk| before the factorization and the block's largest (non-negative
     // doubles order like their bit patterns); the factorization has barriers
@@ -991,7 +1093,7 @@ __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ front
             double* X64 = A64 + kNB * LDA;
             ElimBufs<double, kNB, true>& s64 = *reinterpret_cast<ElimBufs<double, kNB, true>*>(sraw);
             __syncthreads();
-            diag_block_load<double, T>(A64, X64, Pj, ld, c0, w);
+            diag_block_load<double, T, true>(A64, X64, Pj, ld, c0, w);
             __syncthreads();
             bad = diag_block<double, LDLT, false>(A64, X64, s64, w, signs, (int64_t)f.col0 + c0, reg);
             if (bad < 0) {
@@ -1266,8 +1368,9 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
     double* C = Pj;
     bool tri = true;
     if (ROLE == G_LEFT) {
-        ra = c0 + row0, rb = c0, kbeg = obs, kend = c0;
-        rlo = clo = c0, chi = min(nn, c0 + kNB);
+        const int r0 = min(nn, c0 + kNB);  // k_diag updates the rows above
+        ra = (BM == 128 ? r0 & ~3 : r0) + row0, rb = c0, kbeg = obs, kend = c0;
+        rlo = r0, clo = c0, chi = r0, tri = false;
     } else if (ROLE == G_TRAIL) {
         const int e = min(nn, obs + obw);
         const int cs = e + it.b * (PAIR ? 2 * kTile : kTile);
@@ -1291,7 +1394,10 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
     // past the rows, or wholly above the diagonal (the wait is still taken: the
     // next grid may rely on the one before this)
     const bool none = ra >= rhi || (tri && ra + BM <= rb);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // LEFT runs beside k_diag, which let it launch once the grids before had
+    // completed, and waits for it at the end: the TRSM relies on both
+    auto wait = []() { asm volatile("griddepcontrol.wait;" ::: "memory"); };
+    if (none || ROLE != G_LEFT) wait();
     if (none) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int WM = g64_wm<BM>(), MI = WM / 8;
@@ -1392,6 +1498,7 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
                 C[row + (int64_t)col * ldc] = v;
             }
     }
+    if (ROLE == G_LEFT) wait();
 }
 
 // ---------------------------------------------------------------------------
@@ -1724,7 +1831,10 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
                                  kWarpFronts * warp_slice<kWarpSmallNJ>()));
     MF_CUDA(cudaFuncSetAttribute(k_small_warp<T, LDLT, kWarpSmallNJ2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kWarpFronts * warp_slice<kWarpSmallNJ2>()));
-    MF_CUDA(cudaFuncSetAttribute(k_diag<T, LDLT, REG>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<T>()));
+    // sub-panels after an outer block's first: the diagonal block's update in k_diag (FP64), or in LEFT's first tile
+    constexpr bool upd = std::is_same<T, double>::value;
+    MF_CUDA(cudaFuncSetAttribute(k_diag<T, LDLT, REG, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<T>()));
+    MF_CUDA(cudaFuncSetAttribute(k_diag<T, LDLT, REG, upd>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<T>()));
     MF_CUDA(cudaFuncSetAttribute(k_inv256<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, inv256_smem<T>()));
     const Item* items = h->d_items;
     // per-level timing while autotuning (profile mode: no graph, synchronised)
@@ -1813,6 +1923,11 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
         for (const PanelStep& st : lv.steps) {
             const int obs = st.b * lv.kob, obw = lv.kob;
             const int c0 = obs + st.s * kNB;
+            auto launch_diag = [&](auto update) {
+                launch_kx(h->panel_pdl || pdl_enabled(), k_diag<T, LDLT, REG, decltype(update)::value>,
+                          grid_for(st.diag.cnt), 256, diag_smem<T>(), h->stream, h->d_fronts, items + st.diag.off, obs,
+                          c0, fb.P, fb.inv, fb.d, h->d_signs, h->d_info, h->d_rescued, reg);
+            };
             if (std::is_same<T, float>::value && h->use_tc && lv.tc_steps) {
                 // single precision: the GEMM roles run on the tcgen05 tensor cores
                 const FactorBufs<float>& f32b = reinterpret_cast<const FactorBufs<float>&>(fb);
@@ -1823,9 +1938,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
                 }
                 if (st.diag.cnt) {
                     Timer t(h, K_DIAG);
-                    launch_kx(h->panel_pdl || pdl_enabled(), k_diag<T, LDLT, REG>, grid_for(st.diag.cnt), 256,
-                        diag_smem<T>(), h->stream, h->d_fronts, items + st.diag.off, c0, fb.P, fb.inv, fb.d,
-                        h->d_signs, h->d_info, h->d_rescued, reg);
+                    launch_diag(std::false_type{});
                     MF_CUDA(cudaGetLastError());
                 }
                 if (st.panel_tc.cnt) {
@@ -1851,16 +1964,19 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
                 }
                 continue;
             }
-            if (st.left.cnt) {
+            if (!upd && st.left.cnt) {
                 Timer t(h, K_LEFT);
                 if (int rc = gemm_role<T, G_LEFT, LDLT>(h, st.left, st.left_tc, obs, obw, c0, fb)) return rc;
             }
             if (st.diag.cnt) {
                 Timer t(h, K_DIAG);
-                launch_kx(h->panel_pdl || pdl_enabled(), k_diag<T, LDLT, REG>, grid_for(st.diag.cnt), 256,
-                    diag_smem<T>(), h->stream, h->d_fronts, items + st.diag.off, c0, fb.P, fb.inv, fb.d,
-                    h->d_signs, h->d_info, h->d_rescued, reg);
+                if (st.s > 0) launch_diag(std::bool_constant<upd>{});
+                else launch_diag(std::false_type{});
                 MF_CUDA(cudaGetLastError());
+            }
+            if (upd && st.s > 0 && st.panel.cnt) {
+                Timer t(h, K_LEFT);
+                if (int rc = gemm_role<T, G_LEFT, LDLT>(h, st.panel, st.panel_tc, obs, obw, c0, fb)) return rc;
             }
             if (st.panel.cnt) {
                 Timer t(h, K_PANEL);

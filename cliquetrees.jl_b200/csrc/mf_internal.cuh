@@ -130,7 +130,10 @@ constexpr int64_t kMidMaxL21 = 1 << 20;  // such levels' largest nn * na (a clus
 // One 64-wide sub-panel s of outer block b (columns b*kob + s*kNB ..., kob the level's outer-block width).
 struct PanelStep {
     int b = 0, s = 0;
-    ItemList left;    // (front, row tile)  : left-looking update from the outer block's earlier sub-panels
+    // (front, row tile): left-looking update from the outer block's earlier
+    // sub-panels (single precision; in FP64 k_diag updates the diagonal block
+    // and the rows below go by the panel lists)
+    ItemList left;
     ItemList diag;    // (front)            : diagonal block factor + inverse
     ItemList panel;   // (front, row tile)  : panel TRSM below the diagonal block (GEMM with the inverse)
     ItemList trail;   // (front, ti, tj)    : after the last sub-panel of an outer block: trailing update, K = kob
