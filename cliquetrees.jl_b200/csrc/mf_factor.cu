@@ -545,7 +545,7 @@ constexpr int kSmallRescue = 67;
 template <typename T, int LDLT, int TD, int R, bool REG>
 __global__ void __launch_bounds__(TD * TD) k_small(const Front* __restrict__ fronts, const Item* __restrict__ items,
                                                    int stage, const int32_t* __restrict__ reltgt,
-                                                   const int32_t* __restrict__ chdtgt, T* P, T* M, T* __restrict__ d,
+                                                   const int32_t* __restrict__ chdtgt, T* P, T* M, T* d,
                                                    const double* __restrict__ signs, long long* __restrict__ info,
                                                    int* __restrict__ rescued, Reg reg) {
     pdl_trigger();
@@ -1044,8 +1044,8 @@ static_assert(kNB * DLD <= kNB * LDA + 4 * kNB, "the stage ends inside the elimi
 // reported through info.
 template <typename T, int LDLT, bool REG, bool UPDATE>
 __global__ void __launch_bounds__(256, 1) k_diag(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                              int obs, int c0, T* P, T* __restrict__ inv,
-                                              T* __restrict__ d, const double* __restrict__ signs,
+                                              int obs, int c0, T* P, T* inv,
+                                              T* d, const double* __restrict__ signs,
                                               long long* __restrict__ info, int* __restrict__ rescued, Reg reg) {
     if (!UPDATE) pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1245,8 +1245,7 @@ enum GemmRole { G_LEFT = 0, G_TRAIL = 1, G_SYRK = 2, G_TRSM = 3 };
 
 template <typename T, int ROLE, int LDLT>
 __global__ void __launch_bounds__(256) k_gemm(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                              int obs, int obw, int c0, T* __restrict__ P, T* __restrict__ M,
-                                              const T* __restrict__ d, const T* __restrict__ inv) {
+                                              int obs, int obw, int c0, T* P, T* M, const T* d, const T* inv) {
     pdl_prologue();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* smem = reinterpret_cast<T*>(smem_raw);
@@ -1346,8 +1345,8 @@ __device__ __forceinline__ void g64_copy(double* dst, const double* src, int64_t
 template <int BM, int ROLE, int LDLT>
 __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64(const Front* __restrict__ fronts,
                                                                  const Item* __restrict__ items, int obs, int obw,
-                                                                 int c0, double* P, double* M, const double* __restrict__ d,
-                                                                 const double* __restrict__ inv) {
+                                                                 int c0, double* P, double* M, const double* d,
+                                                                 const double* inv) {
     pdl_trigger();
     constexpr int NT = g64_threads<BM>(), LA = BM + 4, LB = kTile + 4, STG = g64_stage<BM>();
     constexpr bool PAIR = BM == 128 && (ROLE == G_TRAIL || ROLE == G_SYRK);

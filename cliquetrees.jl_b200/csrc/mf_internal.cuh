@@ -462,6 +462,12 @@ inline bool pdl_enabled() {
     return on;
 }
 
+// A kernel launched with the attribute may be resident while the grids before
+// it still write.  Memory that any of those grids writes (panels, update
+// matrices, pivots, inverses, split operands, vectors) is therefore never
+// __restrict__ in its parameters: that promises memory which nobody else
+// changes during the kernel, so a read of it could be moved over the wait or
+// served by the read-only path.
 // the launch itself: with the attribute when `pdl`
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kx(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,

@@ -808,8 +808,8 @@ __device__ __forceinline__ void sdiag_run(const Front& f, int step, int q, const
 
 template <typename T, int NR, int BWD>
 __global__ void __launch_bounds__(256) k_s_sdiag(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                                 int step, const T* __restrict__ inv2, T* __restrict__ C,
-                                                 const T* __restrict__ W, int64_t n, int nrhs) {
+                                                 int step, const T* __restrict__ inv2, T* C, const T* W, int64_t n,
+                                                 int nrhs) {
     pdl_trigger();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     const Front f = fronts[items[blockIdx.x / kDiagSplit].front];
@@ -942,8 +942,8 @@ __device__ __forceinline__ void ftile_run(const Front& f, int step, int ta, cons
 
 template <typename T, int NR>
 __global__ void __launch_bounds__(256) k_s_ftile(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                                 int step, const T* __restrict__ P, const T* __restrict__ C,
-                                                 T* __restrict__ W, int64_t n, int nrhs) {
+                                                 int step, const T* __restrict__ P, const T* C, T* W, int64_t n,
+                                                 int nrhs) {
     pdl_trigger();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     const Item it = items[blockIdx.x];
@@ -1176,8 +1176,8 @@ __device__ __forceinline__ void btile_run(const Front& f, int step, int ta, cons
 
 template <typename T, int NR>
 __global__ void __launch_bounds__(256) k_s_btile(const Front* __restrict__ fronts, const Item* __restrict__ items,
-                                                 int step, const T* __restrict__ P, const T* __restrict__ C,
-                                                 T* __restrict__ W, int64_t n, int nrhs) {
+                                                 int step, const T* __restrict__ P, const T* C, T* W, int64_t n,
+                                                 int nrhs) {
     pdl_trigger();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     const Item it = items[blockIdx.x];

@@ -323,11 +323,10 @@ __device__ __forceinline__ TileGeom tile_geom(const Front* __restrict__ fronts, 
 template <int ROLE, int LDLT, bool SPLIT>
 __global__ void __launch_bounds__(tc::NT, 1) k_gemm_tc(const Front* __restrict__ fronts,
                                                        const Item* __restrict__ items, int64_t ntiles, int obs, int obw, int c0,
-                                                       float* P, float* M,
-                                                       const float* __restrict__ d,
+                                                       float* P, float* M, const float* d,
                                                        const CUtensorMap* __restrict__ maps,
                                                        const CUtensorMap* __restrict__ inv_map,
-                                                       const float* __restrict__ split, int* __restrict__ err) {
+                                                       const float* split, int* __restrict__ err) {
     pdl_trigger();
     using namespace tc;
     constexpr int TN = TcTileN<ROLE>::value;
