@@ -1031,7 +1031,7 @@ static_assert(kNB * DLD <= kNB * LDA + 4 * kNB, "the stage ends inside the elimi
 // after its own wait, when all that both read is complete, and LEFT waits for
 // this kernel at its end.  KKT 24 10.78 -> 10.30 ms (a sub-panel's update and
 // block 25 -> 23 us, and its rows' update off the chain), 80^3 81.1 -> 79.3,
-// 16^3 1.182 -> 1.168 ms.
+// 16^3 1.182 -> 1.168 ms.  (diag_and_left in factor_impl launches the pair.)
 // Not in single precision: on the chain the update costs the 64 x 64 x K
 // products on one SM, about what the tensor-core launch took (KKT 24 mixed
 // 9.08 -> 9.04 ms, 80^3 mixed 32.65 -> 32.80, 512^2 8.56 -> 8.55).
@@ -1317,13 +1317,35 @@ constexpr int g64_wm() { return BM == 32 ? 16 : 32; }  // rows per warp
 template <int BM>
 constexpr int g64_threads() { return 32 * (BM / g64_wm<BM>()) * (kTile / 32); }
 
+__device__ __forceinline__ double ld_l2(const double* p) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];\n" : "=d"(v) : "l"(p));
+    return v;
+}
+
 // copy rows [row0, row0 + ROWS) x columns [k, k + GK) of a column-major matrix
 // into dst[kk * (ROWS + 4) + m]; rows at or past rlim (rounded up to the next
-// even one) and columns at or past kend become zeros
-template <int ROWS, int NT, bool VEC>
+// even one) and columns at or past kend become zeros.  L2: nothing is read
+// through L1 (an 8-byte asynchronous copy would be)
+template <int ROWS, int NT, bool VEC, bool L2>
 __device__ __forceinline__ void g64_copy(double* dst, const double* src, int64_t ld, int row0, int rlim, int k, int kend) {
     constexpr int W = VEC ? 2 : 1, PER = ROWS / W;
     static_assert((GK * PER) % NT == 0, "whole rounds of copies");
+    if constexpr (L2 && !VEC) {
+        double v[GK * PER / NT];
+#pragma unroll
+        for (int u = 0; u < GK * PER / NT; ++u) {
+            const int i = threadIdx.x + u * NT, m = i % PER, kk = i / PER;
+            const bool ok = row0 + m < rlim && k + kk < kend;
+            v[u] = ok ? ld_l2(src + (row0 + m) + (int64_t)(k + kk) * ld) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < GK * PER / NT; ++u) {
+            const int i = threadIdx.x + u * NT;
+            dst[i / PER * (ROWS + 4) + i % PER] = v[u];
+        }
+        return;
+    }
 #pragma unroll
     for (int u = 0; u < GK * PER / NT; ++u) {
         const int i = threadIdx.x + u * NT;
@@ -1393,8 +1415,14 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
     // past the rows, or wholly above the diagonal (the wait is still taken: the
     // next grid may rely on the one before this)
     const bool none = ra >= rhi || (tri && ra + BM <= rb);
-    // LEFT runs beside k_diag, which let it launch once the grids before had
-    // completed, and waits for it at the end: the TRSM relies on both
+    // LEFT runs beside the k_diag<UPDATE> that is launched directly before it
+    // (diag_and_left): that kernel lets it go only once its own wait has shown
+    // that the grids before are complete, and so that what they wrote is in
+    // L2.  This SM's L1 may still hold lines from before those writes, which
+    // only a wait of this grid's own would drop, so LEFT reads panels and
+    // pivots through L2 alone.  It waits for k_diag at its end: the TRSM
+    // relies on both.
+    constexpr bool L2 = ROLE == G_LEFT;
     auto wait = []() { asm volatile("griddepcontrol.wait;" ::: "memory"); };
     if (none || ROLE != G_LEFT) wait();
     if (none) return;
@@ -1405,18 +1433,24 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
     const double* dj = (LDLT && ROLE != G_TRSM) ? d + f.col0 : nullptr;
     const bool vec = ((ra | rb) & 1) == 0;
     const int nchunk = (kend - kbeg + GK - 1) / GK;
+    double dn = 0.0;
+    if (LDLT && L2 && tid < GK && kbeg + tid < kend) dn = ld_l2(dj + kbeg + tid);
     auto load = [&](int c) {
         if (c < nchunk) {
             double* st = smem + (c % GStages) * STG;
             const int k = kbeg + c * GK;
             if (vec) {
-                g64_copy<BM, NT, true>(st, Pj, ld, ra, nj, k, kend);
-                g64_copy<kTile, NT, true>(st + GK * LA, Bm, ldb, rb, blim, k, kend);
+                g64_copy<BM, NT, true, L2>(st, Pj, ld, ra, nj, k, kend);
+                g64_copy<kTile, NT, true, L2>(st + GK * LA, Bm, ldb, rb, blim, k, kend);
             } else {
-                g64_copy<BM, NT, false>(st, Pj, ld, ra, nj, k, kend);
-                g64_copy<kTile, NT, false>(st + GK * LA, Bm, ldb, rb, blim, k, kend);
+                g64_copy<BM, NT, false, L2>(st, Pj, ld, ra, nj, k, kend);
+                g64_copy<kTile, NT, false, L2>(st + GK * LA, Bm, ldb, rb, blim, k, kend);
             }
-            if (LDLT && ROLE != G_TRSM && tid < GK) {
+            if (LDLT && L2 && tid < GK) {
+                st[GK * (LA + LB) + tid] = dn;  // fetched a stage ahead
+                const int kn = k + GK + tid;
+                dn = kn < kend ? ld_l2(dj + kn) : 0.0;
+            } else if (LDLT && ROLE != G_TRSM && tid < GK) {
                 const bool ok = k + tid < kend;
                 const unsigned sd = (unsigned)__cvta_generic_to_shared(st + GK * (LA + LB) + tid);
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sd), "l"(dj + (ok ? k + tid : 0)),
@@ -1479,7 +1513,9 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
             for (int e = 0; e < 2; ++e) {
                 const int col = (ROLE == G_TRSM ? c0 : rb) + wc + j * 8 + fk * 2 + e;
                 const bool ok = rok && col >= clo && col < chi && (!tri || row >= col);
-                cv[j][e] = (ok && (ROLE == G_LEFT || ROLE == G_TRAIL)) ? C[row + (int64_t)col * ldc] : 0.0;
+                cv[j][e] = 0.0;
+                if (ok && L2) cv[j][e] = ld_l2(C + row + (int64_t)col * ldc);
+                else if (ok && ROLE == G_TRAIL) cv[j][e] = C[row + (int64_t)col * ldc];
             }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -1967,15 +2003,25 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
                 Timer t(h, K_LEFT);
                 if (int rc = gemm_role<T, G_LEFT, LDLT>(h, st.left, st.left_tc, obs, obw, c0, fb)) return rc;
             }
-            if (st.diag.cnt) {
-                Timer t(h, K_DIAG);
-                if (st.s > 0) launch_diag(std::bool_constant<upd>{});
-                else launch_diag(std::false_type{});
-                MF_CUDA(cudaGetLastError());
-            }
-            if (upd && st.s > 0 && st.panel.cnt) {
+            // FP64: the block's update, factor and inverse, and LEFT beside it.
+            // LEFT takes no wait before it reads (see k_gemm64), so nothing
+            // may come between the two, and LEFT follows no other kernel
+            auto diag_and_left = [&]() -> int {
+                {
+                    Timer t(h, K_DIAG);
+                    launch_diag(std::bool_constant<upd>{});
+                    MF_CUDA(cudaGetLastError());
+                }
+                if (!st.panel.cnt) return 0;
                 Timer t(h, K_LEFT);
-                if (int rc = gemm_role<T, G_LEFT, LDLT>(h, st.panel, st.panel_tc, obs, obw, c0, fb)) return rc;
+                return gemm_role<T, G_LEFT, LDLT>(h, st.panel, st.panel_tc, obs, obw, c0, fb);
+            };
+            if (upd && st.s > 0) {
+                if (int rc = diag_and_left()) return rc;
+            } else if (st.diag.cnt) {
+                Timer t(h, K_DIAG);
+                launch_diag(std::false_type{});
+                MF_CUDA(cudaGetLastError());
             }
             if (st.panel.cnt) {
                 Timer t(h, K_PANEL);
