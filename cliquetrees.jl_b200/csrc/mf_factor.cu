@@ -1791,7 +1791,7 @@ int launch_panel32_to_dl(mf_handle* h, double* dD, double* dL) {
 template <int BM, int ROLE, int LDLT>
 static int gemm64_go(mf_handle* h, int64_t ctas, const Item* items, int obs, int obw, int c0,
                      const FactorBufs<double>& fb) {
-    const bool pdl = pdl_enabled() || (h->panel_pdl && ROLE != G_TRAIL);
+    const bool pdl = early(h, pdl_enabled() || (h->panel_pdl && ROLE != G_TRAIL));
     MF_CUDA(cudaFuncSetAttribute(k_gemm64<BM, ROLE, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, g64_smem<BM>()));
     launch_kx(pdl, k_gemm64<BM, ROLE, LDLT>, grid_for(ctas), g64_threads<BM>(), g64_smem<BM>(), h->stream, h->d_fronts,
               items, obs, obw, c0, fb.P, fb.M, fb.d, fb.inv);
@@ -1823,7 +1823,7 @@ static int gemm_role(mf_handle* h, const ItemList& small, const ItemList& large,
     } else {
         constexpr int gs = gemm_smem<T>();
         MF_CUDA(cudaFuncSetAttribute(k_gemm<T, ROLE, LDLT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs));
-        launch_kx(pdl_enabled() || (h->panel_pdl && (ROLE == G_LEFT || ROLE == G_TRSM)), k_gemm<T, ROLE, LDLT>,
+        launch_kx(early(h, pdl_enabled() || (h->panel_pdl && (ROLE == G_LEFT || ROLE == G_TRSM))), k_gemm<T, ROLE, LDLT>,
                   grid_for(small.cnt), 256, gs, h->stream, h->d_fronts, h->d_items + small.off, obs, obw, c0, fb.P, fb.M,
                   fb.d, fb.inv);
         MF_CUDA(cudaGetLastError());
@@ -1842,7 +1842,7 @@ static int small_go(mf_handle* h, const ItemList& l, int mj, int stage, const Fa
     const size_t sm = std::max<size_t>(((size_t)stage + (size_t)lj * mj) * sizeof(T), sizeof(T) == 4 ? (size_t)rj * rj * 8 : 0);
     MF_CUDA(cudaFuncSetAttribute(k_small<T, LDLT, TD, R, REG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (kSmallStage + kSmallMax * kSmallMax) * (int)sizeof(T)));
-    launch_kx(h->panel_pdl || pdl_enabled(), k_small<T, LDLT, TD, R, REG>, grid_for(l.cnt), TD * TD, sm, h->stream, h->d_fronts,
+    launch_kx(early(h, h->panel_pdl || pdl_enabled()), k_small<T, LDLT, TD, R, REG>, grid_for(l.cnt), TD * TD, sm, h->stream, h->d_fronts,
              h->d_items + l.off, stage, h->d_reltgt, h->d_chdtgt, fb.P, fb.M, fb.d, h->d_signs, h->d_info,
              h->d_rescued, reg);
     MF_CUDA(cudaGetLastError());
@@ -1879,6 +1879,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
         h->tune_steps_ms.assign(h->levels.size(), 0.0);
         h->tune_syrk_ms.assign(h->levels.size(), 0.0);
     }
+    h->seq_begun = false;
     for (size_t L = 0; L < h->levels.size(); ++L) {
         const Level& lv = h->levels[L];
         if (lv.small_warp.cnt) {
@@ -1898,6 +1899,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
                 reg);
             MF_CUDA(cudaGetLastError());
         }
+        if (lv.small_warp.cnt || lv.small_warp2.cnt) h->seq_begun = true;
         if (lv.small.cnt) {
             Timer t(h, K_SMALL);
             // one launch sized for the level's largest front; a level that
@@ -1920,7 +1922,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
         }
         if (lv.ea.cnt) {
             Timer t(h, K_EA);
-            launch_kx(h->panel_pdl || pdl_enabled(), k_ea<T, 0>, grid_for(lv.ea.cnt), 256, 0, h->stream, h->d_fronts, items + lv.ea.off, items,
+            launch_kx(early(h, h->panel_pdl || pdl_enabled()), k_ea<T, 0>, grid_for(lv.ea.cnt), 256, 0, h->stream, h->d_fronts, items + lv.ea.off, items,
                                                                    h->d_reltgt, fb.P, fb.M);
             MF_CUDA(cudaGetLastError());
         }
@@ -1959,7 +1961,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
             const int obs = st.b * lv.kob, obw = lv.kob;
             const int c0 = obs + st.s * kNB;
             auto launch_diag = [&](auto update) {
-                launch_kx(h->panel_pdl || pdl_enabled(), k_diag<T, LDLT, REG, decltype(update)::value>,
+                launch_kx(early(h, h->panel_pdl || pdl_enabled()), k_diag<T, LDLT, REG, decltype(update)::value>,
                           grid_for(st.diag.cnt), 256, diag_smem<T>(), h->stream, h->d_fronts, items + st.diag.off, obs,
                           c0, fb.P, fb.inv, fb.d, h->d_signs, h->d_info, h->d_rescued, reg);
             };
@@ -2061,7 +2063,7 @@ static int factor_impl(mf_handle* h, const FactorBufs<T>& fb) {
         }
         if (lv.ea_upd.cnt) {
             Timer t(h, K_EA);
-            launch_kx(h->panel_pdl || pdl_enabled(), k_ea<T, 1>, grid_for(lv.ea_upd.cnt), 256, 0, h->stream, h->d_fronts, items + lv.ea_upd.off, items,
+            launch_kx(early(h, h->panel_pdl || pdl_enabled()), k_ea<T, 1>, grid_for(lv.ea_upd.cnt), 256, 0, h->stream, h->d_fronts, items + lv.ea_upd.off, items,
                                                                        h->d_reltgt, fb.P, fb.M);
             MF_CUDA(cudaGetLastError());
         }

@@ -357,6 +357,7 @@ struct mf_handle {
     bool panel_pdl = true;         // the factorization's short launches (small fronts, extend-add, left-looking,
                                    // diagonal block, TRSM, SYRK) launched for programmatic dependence: setup
                                    // and static loads beside the launch before (MF_PANEL_PDL=0: off)
+    bool seq_begun = false;        // the launch sequence being queued has made its first launch (early())
     cudaStream_t side = nullptr;   // the factorization's look-ahead stream (trailing updates beside the next
                                    // outer block's sub-panels), forked from and joined into `stream`
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -440,15 +441,34 @@ void set_error(const std::string& msg);
 std::recursive_mutex& device_mutex();
 int cuda_fail(cudaError_t e, const char* where);
 
-// Programmatic dependent launch.  Every kernel of the factorization, solve
-// and refinement paths starts with pdl_prologue(): it waits until the grid
-// it depends on has completed and its memory is visible (a no-op for a grid
-// launched without the attribute), then lets the next grid of the stream be
-// launched.  launch_k() launches with the attribute, so consecutive kernels
-// of a captured graph overlap the next launch's setup with the tail of the
-// current one while keeping stream order for every memory access.  Opt-in
-// (MF_PDL=1 in the environment): on the 80^3 workload the graph replays ran
-// about 2 % slower with it (100.9 vs 98.8 ms FP64, 46.9 vs 45.9 ms mixed).
+// Programmatic dependent launch.  A grid launched with the attribute becomes
+// resident once every CTA of the grid before it has let it go (or ended); its
+// griddepcontrol.wait returns when that grid has completed and its memory is
+// visible.  Every kernel takes the wait in every CTA, so a grid that is past
+// its wait has everything queued before it complete.  The wait is a no-op for a
+// grid launched without the attribute, which starts after the one before it.
+//
+// Kernels that wait first and then let the next grid go (pdl_prologue): all but
+// the following.  These let it go at their start (pdl_trigger) and read, before
+// their wait, only what no launch of their own sequence has yet written:
+//   factorization (attribute unless MF_PANEL_PDL=0)
+//     k_small      the front's assembled panel and the children's records
+//     k_ea         segments, records and relative indices of the children
+//     k_diag       nothing; with UPDATE it lets the next grid go after its wait
+//     k_gemm64     nothing; LEFT takes its wait at the end (see diag_and_left)
+//     k_gemm_tc    nothing (barriers and tensor memory are set up)
+//   solves (attribute unless MF_STEP_PDL=0), which write no factor
+//     k_s_cta_fwd, k_s_cta_bwd, k_s_ftile, k_s_btile   panels
+//     k_s_fwd_l, k_s_bwd_l                             panels (early_panel())
+//     k_s_sdiag                                        super-block inverses
+//     k_s_gather                                       contribution lists
+// k_gemm (LEFT, TRSM), k_s_fwd_red and k_s_bwd_red are launched with the
+// attribute too but wait first.  early() below keeps the first launch of a
+// sequence from starting before the work queued ahead of it is complete.
+//
+// MF_PDL=1 in the environment launches every kernel with the attribute: on the
+// 80^3 workload the graph replays ran about 2 % slower with it (100.9 vs 98.8 ms
+// FP64, 46.9 vs 45.9 ms mixed).
 __device__ __forceinline__ void pdl_prologue() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -485,18 +505,26 @@ inline cudaError_t launch_kx(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 b
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
+// Whether the next launch of a factorization or solve may start early (with the
+// attribute; `want` is the kernel's own choice).  The sequence's first may not:
+// it waits for everything queued before the sequence, and with that every later
+// launch starts after it.  So any of them may read, before its own wait, what
+// was complete when the sequence was queued: a factorization's k_small the
+// assembled panels (k_scatter lets its successor go before it writes them), a
+// solve the factor.  The sequence itself must not write it earlier on, of course.
+inline bool early(mf_handle* h, bool want) {
+    const bool ok = h->seq_begun && want;
+    h->seq_begun = true;
+    return ok;
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                             Args&&... args) {
     return launch_kx(pdl_enabled(), kern, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
-// The blocked solve-step kernels (k_s_sdiag, k_s_ftile, k_s_btile) let the
-// next grid launch at once and wait for the previous one only after they
-// have issued their loads of the panel or the inverse, which no kernel of
-// the solve writes; they are launched with the attribute unless
-// MF_STEP_PDL=0, so each step's launch and those loads overlap the step
-// before it.
+// lets the next grid of the stream be launched at once; the kernel's own wait comes later
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 

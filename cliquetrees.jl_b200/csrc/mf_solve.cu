@@ -1816,6 +1816,7 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
         MF_CUDA(cudaGetLastError());
     }
     // forward: levels ascending
+    h->seq_begun = h->sub_tasks.cnt > 0;
     for (const Level& lv : h->levels) {
         if (lv.s_cta.items.cnt)
             if (int rc = launch_solve_cta(h, lv, sb, 0, nrb, nrhs)) return rc;
@@ -1850,7 +1851,7 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
         }
         if (lv.s_gather.cnt) {
             Timer t(h, K_S_GATHER);
-            launch_kx(h->step_pdl, k_s_gather<T>, (unsigned)lv.s_gather.cnt, 256, 0, h->stream, 
+            launch_kx(early(h, h->step_pdl), k_s_gather<T>, (unsigned)lv.s_gather.cnt, 256, 0, h->stream, 
                 h->d_fronts, items + lv.s_gather.off, h->d_grow, h->d_gcon, sb.C, sb.W, sb.R, n, nrhs);
             MF_CUDA(cudaGetLastError());
         }
@@ -1866,22 +1867,22 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
             const unsigned gd = (unsigned)st.diag.cnt;
             const Item* itd = items + st.diag.off;
             switch (nrb) {
-                case 1: launch_kx(h->step_pdl, k_s_sdiag<T, 1, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 1>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
-                case 2: launch_kx(h->step_pdl, k_s_sdiag<T, 2, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 2>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
-                case 4: launch_kx(h->step_pdl, k_s_sdiag<T, 4, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 4>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
-                case 8: launch_kx(h->step_pdl, k_s_sdiag<T, 8, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 8>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
-                default: launch_kx(h->step_pdl, k_s_sdiag<T, 16, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 16>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                case 1: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 1, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 1>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                case 2: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 2, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 2>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                case 4: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 4, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 4>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                case 8: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 8, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 8>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                default: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 16, 0>, gd * kDiagSplit, 256, sdiag_smem<T, 16>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
             }
             MF_CUDA(cudaGetLastError());
             if (st.fwd.cnt) {
                 const unsigned gf = (unsigned)st.fwd.cnt;
                 const Item* itf = items + st.fwd.off;
                 switch (nrb) {
-                    case 1: launch_kx(h->step_pdl, k_s_ftile<T, 1>, gf, 256, ftile_smem<T, 1>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
-                    case 2: launch_kx(h->step_pdl, k_s_ftile<T, 2>, gf, 256, ftile_smem<T, 2>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
-                    case 4: launch_kx(h->step_pdl, k_s_ftile<T, 4>, gf, 256, ftile_smem<T, 4>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
-                    case 8: launch_kx(h->step_pdl, k_s_ftile<T, 8>, gf, 256, ftile_smem<T, 8>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
-                    default: launch_kx(h->step_pdl, k_s_ftile<T, 16>, gf, 256, ftile_smem<T, 16>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    case 1: launch_kx(early(h, h->step_pdl), k_s_ftile<T, 1>, gf, 256, ftile_smem<T, 1>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    case 2: launch_kx(early(h, h->step_pdl), k_s_ftile<T, 2>, gf, 256, ftile_smem<T, 2>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    case 4: launch_kx(early(h, h->step_pdl), k_s_ftile<T, 4>, gf, 256, ftile_smem<T, 4>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    case 8: launch_kx(early(h, h->step_pdl), k_s_ftile<T, 8>, gf, 256, ftile_smem<T, 8>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    default: launch_kx(early(h, h->step_pdl), k_s_ftile<T, 16>, gf, 256, ftile_smem<T, 16>(), h->stream, h->d_fronts, itf, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
                 }
                 MF_CUDA(cudaGetLastError());
             }
@@ -1891,14 +1892,14 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
             const unsigned gl = (unsigned)lv.s_fwd_l.cnt;
             const Item* itl = items + lv.s_fwd_l.off;
             switch (nrb) {
-                case 1: launch_kx(early_panel<T, 1>() && h->step_pdl, k_s_fwd_l<T, 1>, gl, 256, fwdl_smem<T, 1>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
-                case 2: launch_kx(early_panel<T, 2>() && h->step_pdl, k_s_fwd_l<T, 2>, gl, 256, fwdl_smem<T, 2>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
-                case 4: launch_kx(early_panel<T, 4>() && h->step_pdl, k_s_fwd_l<T, 4>, gl, 256, fwdl_smem<T, 4>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
-                case 8: launch_kx(early_panel<T, 8>() && h->step_pdl, k_s_fwd_l<T, 8>, gl, 256, fwdl_smem<T, 8>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
-                default: launch_kx(early_panel<T, 16>() && h->step_pdl, k_s_fwd_l<T, 16>, gl, 256, fwdl_smem<T, 16>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
+                case 1: launch_kx(early(h, early_panel<T, 1>() && h->step_pdl), k_s_fwd_l<T, 1>, gl, 256, fwdl_smem<T, 1>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
+                case 2: launch_kx(early(h, early_panel<T, 2>() && h->step_pdl), k_s_fwd_l<T, 2>, gl, 256, fwdl_smem<T, 2>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
+                case 4: launch_kx(early(h, early_panel<T, 4>() && h->step_pdl), k_s_fwd_l<T, 4>, gl, 256, fwdl_smem<T, 4>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
+                case 8: launch_kx(early(h, early_panel<T, 8>() && h->step_pdl), k_s_fwd_l<T, 8>, gl, 256, fwdl_smem<T, 8>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
+                default: launch_kx(early(h, early_panel<T, 16>() && h->step_pdl), k_s_fwd_l<T, 16>, gl, 256, fwdl_smem<T, 16>(), h->stream, h->d_fronts, itl, sb.P, sb.C, sb.part, sb.R, n, nrhs); break;
             }
             MF_CUDA(cudaGetLastError());
-            if (lv.s_fwd_red.cnt) launch_kx(h->step_pdl, k_s_fwd_red<T>, (unsigned)lv.s_fwd_red.cnt, 256, 0, h->stream, h->d_fronts, items + lv.s_fwd_red.off,
+            if (lv.s_fwd_red.cnt) launch_kx(early(h, h->step_pdl), k_s_fwd_red<T>, (unsigned)lv.s_fwd_red.cnt, 256, 0, h->stream, h->d_fronts, items + lv.s_fwd_red.off,
                                                                               sb.part, sb.R, nrhs);
             MF_CUDA(cudaGetLastError());
         }
@@ -1921,14 +1922,14 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
             const unsigned gl = (unsigned)lv.s_bwd_l.cnt;
             const Item* itl = items + lv.s_bwd_l.off;
             switch (nrb) {
-                case 1: launch_kx(early_panel<T, 1>() && h->step_pdl, k_s_bwd_l<T, 1>, gl, 256, bwd_smem<T, 1>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
-                case 2: launch_kx(early_panel<T, 2>() && h->step_pdl, k_s_bwd_l<T, 2>, gl, 256, bwd_smem<T, 2>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
-                case 4: launch_kx(early_panel<T, 4>() && h->step_pdl, k_s_bwd_l<T, 4>, gl, 256, bwd_smem<T, 4>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
-                case 8: launch_kx(early_panel<T, 8>() && h->step_pdl, k_s_bwd_l<T, 8>, gl, 256, bwd_smem<T, 8>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
-                default: launch_kx(early_panel<T, 16>() && h->step_pdl, k_s_bwd_l<T, 16>, gl, 256, bwd_smem<T, 16>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 1: launch_kx(early(h, early_panel<T, 1>() && h->step_pdl), k_s_bwd_l<T, 1>, gl, 256, bwd_smem<T, 1>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 2: launch_kx(early(h, early_panel<T, 2>() && h->step_pdl), k_s_bwd_l<T, 2>, gl, 256, bwd_smem<T, 2>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 4: launch_kx(early(h, early_panel<T, 4>() && h->step_pdl), k_s_bwd_l<T, 4>, gl, 256, bwd_smem<T, 4>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 8: launch_kx(early(h, early_panel<T, 8>() && h->step_pdl), k_s_bwd_l<T, 8>, gl, 256, bwd_smem<T, 8>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                default: launch_kx(early(h, early_panel<T, 16>() && h->step_pdl), k_s_bwd_l<T, 16>, gl, 256, bwd_smem<T, 16>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
             }
             MF_CUDA(cudaGetLastError());
-            if (lv.s_bwd_red.cnt) launch_kx(h->step_pdl, k_s_bwd_red<T>, (unsigned)lv.s_bwd_red.cnt, 256, 0, h->stream, h->d_fronts, items + lv.s_bwd_red.off,
+            if (lv.s_bwd_red.cnt) launch_kx(early(h, h->step_pdl), k_s_bwd_red<T>, (unsigned)lv.s_bwd_red.cnt, 256, 0, h->stream, h->d_fronts, items + lv.s_bwd_red.off,
                                                                               sb.part, sb.C, sb.W, n, nrhs);
             MF_CUDA(cudaGetLastError());
         }
@@ -1944,22 +1945,22 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
             const unsigned gd = (unsigned)st.diag.cnt;
             const Item* itd = items + st.diag.off;
             switch (nrb) {
-                case 1: launch_kx(h->step_pdl, k_s_sdiag<T, 1, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 1>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
-                case 2: launch_kx(h->step_pdl, k_s_sdiag<T, 2, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 2>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
-                case 4: launch_kx(h->step_pdl, k_s_sdiag<T, 4, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 4>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
-                case 8: launch_kx(h->step_pdl, k_s_sdiag<T, 8, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 8>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
-                default: launch_kx(h->step_pdl, k_s_sdiag<T, 16, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 16>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                case 1: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 1, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 1>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                case 2: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 2, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 2>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                case 4: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 4, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 4>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                case 8: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 8, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 8>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
+                default: launch_kx(early(h, h->step_pdl), k_s_sdiag<T, 16, 1>, gd * kDiagSplit, 256, sdiag_smem<T, 16>(), h->stream, h->d_fronts, itd, (int)k, sb.inv2, sb.C, sb.W, n, nrhs); break;
             }
             MF_CUDA(cudaGetLastError());
             if (st.bwd.cnt) {
                 const unsigned gb = (unsigned)st.bwd.cnt;
                 const Item* itb = items + st.bwd.off;
                 switch (nrb) {
-                    case 1: launch_kx(h->step_pdl, k_s_btile<T, 1>, gb, 256, btile_smem<T, 1>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
-                    case 2: launch_kx(h->step_pdl, k_s_btile<T, 2>, gb, 256, btile_smem<T, 2>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
-                    case 4: launch_kx(h->step_pdl, k_s_btile<T, 4>, gb, 256, btile_smem<T, 4>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
-                    case 8: launch_kx(h->step_pdl, k_s_btile<T, 8>, gb, 256, btile_smem<T, 8>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
-                    default: launch_kx(h->step_pdl, k_s_btile<T, 16>, gb, 256, btile_smem<T, 16>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    case 1: launch_kx(early(h, h->step_pdl), k_s_btile<T, 1>, gb, 256, btile_smem<T, 1>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    case 2: launch_kx(early(h, h->step_pdl), k_s_btile<T, 2>, gb, 256, btile_smem<T, 2>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    case 4: launch_kx(early(h, h->step_pdl), k_s_btile<T, 4>, gb, 256, btile_smem<T, 4>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    case 8: launch_kx(early(h, h->step_pdl), k_s_btile<T, 8>, gb, 256, btile_smem<T, 8>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
+                    default: launch_kx(early(h, h->step_pdl), k_s_btile<T, 16>, gb, 256, btile_smem<T, 16>(), h->stream, h->d_fronts, itb, (int)k, sb.P, sb.C, sb.W, n, nrhs); break;
                 }
                 MF_CUDA(cudaGetLastError());
             }

@@ -285,11 +285,11 @@ int cta_go(mf_handle* h, const CtaList& l, const SolveBufs<T>& sb, int bwd, int 
     const size_t sm = ((size_t)pan + (size_t)l.rows * NR + kSmallMax) * sizeof(T);
     if (!bwd) {
         MF_CUDA(cudaFuncSetAttribute(k_s_cta_fwd<T, UNIT, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-        launch_kx(h->step_pdl, k_s_cta_fwd<T, UNIT, NR>, g, kCtaThreads, sm, h->stream, h->d_fronts, it, pan,
+        launch_kx(early(h, h->step_pdl), k_s_cta_fwd<T, UNIT, NR>, g, kCtaThreads, sm, h->stream, h->d_fronts, it, pan,
                   l.rows, h->d_reltgt, h->d_chdtgt, sb.P, sb.C, sb.R, h->n, nrhs);
     } else {
         MF_CUDA(cudaFuncSetAttribute(k_s_cta_bwd<T, UNIT, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-        launch_kx(h->step_pdl, k_s_cta_bwd<T, UNIT, NR>, g, kCtaThreads, sm, h->stream, h->d_fronts, it, pan,
+        launch_kx(early(h, h->step_pdl), k_s_cta_bwd<T, UNIT, NR>, g, kCtaThreads, sm, h->stream, h->d_fronts, it, pan,
                   l.rows, h->d_septgt, sb.P, sb.C, h->n, nrhs);
     }
     MF_CUDA(cudaGetLastError());
