@@ -150,29 +150,15 @@ constexpr double kRescueSmall = 1e-5;
 constexpr double kRescueGrowth = 1e7;
 constexpr int kSmallKids = 16;  // children whose records k_small fetches up front
 
-// The reciprocal ik that scales the column of an accepted pivot p: 1 / sqrt(p)
-// for Cholesky, 1 / p for LDLt.  The chain of dependent pivots waits for it, so
-// it takes the shortest sequence of full accuracy: in double CUDA's rsqrt (at
-// most 1 ulp off, what the rounded square root and the rounded division after
-// it reach together); in float the hardware's approximation and one
-// Newton-Raphson step (for y^-2 = p or y^-1 = p), dropped by a select where
-// the step's products leave the exponent range.  The stored diagonal entry
-// (sqrt(p), or p) is formed beside the chain.
-template <int LDLT>
-__device__ __forceinline__ float pivot_recip(float p) {
-    float y;
-    if (LDLT) {
-        asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(p));
-        const float z = fmaf(y, fmaf(-p, y, 1.0f), y);
-        return fabsf(y) > 1e-36f && fabsf(y) < 1e36f ? z : y;
-    }
-    asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(p));
-    const float z = fmaf(0.5f * y, fmaf(-(p * y), y, 1.0f), y);
-    return p < 1e36f ? z : y;
-}
-template <int LDLT>
-__device__ __forceinline__ double pivot_recip(double p) {
-    return LDLT ? 1.0 / p : rsqrt(p);
+// The reciprocal ik that scales the column of an accepted pivot p: one over the
+// stored diagonal entry (sqrt(p) for Cholesky, p for LDLt), both correctly
+// rounded.  BLOCK, single-precision Cholesky: the hardware's reciprocal square
+// root (rsqrtf, at most 2 ulp) in the diagonal blocks, whose factor only
+// preconditions the FP64 refinement and whose pivots are one long chain.
+template <int LDLT, bool BLOCK, typename TC>
+__device__ __forceinline__ TC pivot_recip(TC p) {
+    if (BLOCK && !LDLT && sizeof(TC) == 4) return rsqrtf((float)p);
+    return TC(1) / (LDLT ? p : sqrt(p));
 }
 template <typename TC, int LDLT>
 __device__ __forceinline__ TC pivot_stored(TC p) {
@@ -198,17 +184,18 @@ __device__ __forceinline__ TC pivot_stored(TC p) {
 // for LDLt) in the registers of the finished columns: a second group of NR
 // threads solves X's four pivot rows beside the row group, one column each,
 // into rq and X, and the update is the same for A's and X's entries.
-// What bounds it is the chain of pivots (reciprocal square root, scale and
+// What bounds it is the chain of pivots (square root and reciprocal, scale and
 // update within the quad, two barriers around it), then shared-memory reads of
 // the quads in the update (two rows a warp: 128 bytes a cycle and SM).  So
 // nothing else is on the chain, its code is straight-line, and one rolled
 // loop of a few hundred instructions serves all quads: a CTA runs it once, and
 // its instructions come from L2.  64 x 64 block with its inverse, one CTA, per
-// launch: FP64 Cholesky 36 -> 14 us, LDLt 38 -> 19 us, FP32 17.6 -> 10.7 us
-// and 23.4 -> 14.1 us (before: panels of sixteen columns factored by one
-// warp's shuffles, the inverse after them).  A small front's launch in a
-// narrow level: 44 -> 13 us (before: a right-looking loop in shared memory,
-// two divisions an entry, a barrier a column and a memory trip a child).
+// launch (medians over the blocks of a 1,024-column front): FP64 Cholesky 36 ->
+// 23 us, LDLt 36 -> 21 us, FP32 17.7 -> 12.3 us and 21.7 -> 14.9 us (before:
+// panels of sixteen columns factored by one warp's shuffles, the inverse after
+// them).  A small front's launch in a narrow level: 44 -> 12 to 16 us (before: a
+// right-looking loop in shared memory, two divisions an entry, a barrier a
+// column and a memory trip a child).
 // Measured slower: the matrix in shared memory instead of registers (29 us for
 // the FP64 LDLt block: aliased loads and stores wait for one another), the
 // panel one quad ahead of the update in warps of its own (26 us: the panel
@@ -283,7 +270,7 @@ __device__ __forceinline__ int eliminate(TC (&a)[R][R], int nrow, int nel, TC* F
                 if (c > 0) piv = c < nc ? piv : TC(1);
                 raw[c] = piv;
                 // after a rejected pivot the remaining steps run on junk and are discarded
-                const TC ik = pivot_recip<LDLT>(piv);
+                const TC ik = pivot_recip<LDLT, INV>(piv);
                 TC lv = (LDLT && INV && !row) ? v[c] : v[c] * ik;
                 if (c > 0) lv = c < nc ? lv : TC(0);
 #pragma unroll
@@ -497,7 +484,7 @@ __device__ __noinline__ int small_redo(double* F, const Front& f, const Front* _
         const double piv = F[k + k * nj];
         const double s = pivot_sign(signs, LDLT, f.col0 + k);
         if (!pivot_ok(s, piv) || (!LDLT && !(piv > 0.0))) return k;  // uniform across the block
-        const double inv = pivot_recip<LDLT>(piv);
+        const double inv = pivot_recip<LDLT, false>(piv);
         __syncthreads();
         if (tid == 0) F[k + k * nj] = pivot_stored<double, LDLT>(piv);
         for (int i = k + 1 + tid; i < nj; i += nt) F[i + k * nj] *= inv;
@@ -685,7 +672,7 @@ __device__ int warp_front(TC* F, const Front& f, const Front* __restrict__ front
             const double ap = fabs((double)piv);
             if (ap < kRescueSmall * a0 || ap > kRescueGrowth * fmax(a0, 1.0)) *flag = true;
         }
-        const TC inv = pivot_recip<LDLT>(piv);
+        const TC inv = pivot_recip<LDLT, false>(piv);
         __syncwarp();
         if (lane == k) F[k + k * (ROWS + 1)] = pivot_stored<TC, LDLT>(piv);
         if (lane > k && row) F[lane + k * (ROWS + 1)] *= inv;
@@ -1344,19 +1331,19 @@ __device__ __forceinline__ void g64_copy(double* dst, const double* src, int64_t
             const int i = threadIdx.x + u * NT;
             dst[i / PER * (ROWS + 4) + i % PER] = v[u];
         }
-        return;
-    }
+    } else {
 #pragma unroll
-    for (int u = 0; u < GK * PER / NT; ++u) {
-        const int i = threadIdx.x + u * NT;
-        const int m = (i % PER) * W, kk = i / PER;
-        const bool ok = row0 + m < rlim && k + kk < kend;
-        const double* s = src + (ok ? (row0 + m) + (int64_t)(k + kk) * ld : 0);
-        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + kk * (ROWS + 4) + m);
-        if (VEC)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(s), "r"(ok ? 16 : 0) : "memory");
-        else
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(s), "r"(ok ? 8 : 0) : "memory");
+        for (int u = 0; u < GK * PER / NT; ++u) {
+            const int i = threadIdx.x + u * NT;
+            const int m = (i % PER) * W, kk = i / PER;
+            const bool ok = row0 + m < rlim && k + kk < kend;
+            const double* s = src + (ok ? (row0 + m) + (int64_t)(k + kk) * ld : 0);
+            const unsigned d = (unsigned)__cvta_generic_to_shared(dst + kk * (ROWS + 4) + m);
+            if (VEC)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(s), "r"(ok ? 16 : 0) : "memory");
+            else
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(s), "r"(ok ? 8 : 0) : "memory");
+        }
     }
 }
 
