@@ -6,7 +6,14 @@ reciprocal of the stored diagonal entry (sqrt(p) rounded, or p), over the
 exponent range in FP64, and in single precision over what the scaled matrix can
 hold; there the diagonal blocks' Cholesky takes a reciprocal square root of at
 most 2 ulp.  The expected values are numpy's, each operation of which rounds
-correctly, so all but that last one must be equal bit for bit."""
+correctly, so all but that last one must be equal bit for bit.
+
+Order of sums: a pivot's updates in a diagonal block are summed four columns
+at a time before they are subtracted.  With entries in [1, 2) every subtraction
+adds a rounding error of variance 2^-104 / 12, so the 64th pivot of a block has
+an error of sqrt(18 / 12) 2^-52 in the root mean square (fifteen groups, then
+three columns of its own group); subtracted one by one it would be
+sqrt(63 / 12) 2^-52.  The bar lies between, at 1.6 x 2^-52."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -85,3 +92,25 @@ def test_single_precision_reciprocal_pivot(n, m, ldlt):
         assert np.array_equal(L[:, 2, 1], want.astype(np.float64))
     if ldlt:
         assert np.array_equal(d[:, 1], p.astype(np.float64))
+
+
+@pytest.mark.parametrize("ldlt", [False, True])
+def test_block_sums_updates_by_fours(ldlt):
+    n, m, k = 98, 400, 63
+    rng = np.random.default_rng(17)
+    G = rng.uniform(-0.05, 0.05, (m, 64, 64))
+    blocks = np.zeros((m, n, n))
+    blocks[:, np.arange(n), np.arange(n)] = 1.0
+    blocks[:, :64, :64] = np.tril(G, -1) + np.tril(G, -1).transpose(0, 2, 1)
+    blocks[:, np.arange(64), np.arange(64)] = rng.uniform(1.5, 1.9, (m, 64))
+    X = blocks[:, :64, :64].astype(np.longdouble)
+    for j in range(k):
+        col = X[:, j + 1:, j].copy()
+        X[:, j + 1:, j + 1:] -= col[:, :, None] * (col / X[:, j, j][:, None])[:, None, :]
+    want = X[:, k, k]
+    assert want.min() > 1.0 and want.max() < 2.0
+    L, d = factor(blocks, ldlt, False)
+    have = d[:, k] if ldlt else L[:, k, k].astype(np.longdouble) ** 2
+    rms = 2.0 ** 52 * float(np.sqrt(np.mean((have - want) ** 2)))
+    # the stored square root's rounding: variance 2^-104 / 12, times (2 sqrt(p))^2 in its square
+    assert rms <= np.sqrt(1.6 ** 2 + (0 if ldlt else 4 * 1.9 / 12))
