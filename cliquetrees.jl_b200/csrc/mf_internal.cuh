@@ -461,7 +461,7 @@ int cuda_fail(cudaError_t e, const char* where);
 //     k_s_cta_fwd, k_s_cta_bwd, k_s_ftile, k_s_btile   panels
 //     k_s_fwd_l, k_s_bwd_l                             panels (early_panel())
 //     k_s_sdiag                                        super-block inverses
-//     k_s_gather                                       contribution lists
+//     k_s_gather                                       contribution lists (few CTAs or narrow vectors)
 // k_gemm (LEFT, TRSM), k_s_fwd_red and k_s_bwd_red are launched with the
 // attribute too but wait first.  early() below keeps the first launch of a
 // sequence from starting before the work queued ahead of it is complete.

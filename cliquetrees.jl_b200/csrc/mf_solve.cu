@@ -1851,7 +1851,15 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
         }
         if (lv.s_gather.cnt) {
             Timer t(h, K_S_GATHER);
-            launch_kx(early(h, h->step_pdl), k_s_gather<T>, (unsigned)lv.s_gather.cnt, 256, 0, h->stream, 
+            // Early where it has at most a CTA per SM (300^2 FP64, eight
+            // right-hand sides: 1.90 -> 1.86 ms a pass; KKT 24 mixed 9.30 -> 9.24)
+            // or narrow vectors (as early_panel(); 512^2 FP32, four: 8.66 -> 8.53 ms,
+            // 48^3 FP64, two, three overlapping: 0.84 -> 0.80).  Larger launches
+            // with wide vectors hold places while they wait that other
+            // streams' solves could use: three overlapping 48^3 FP64 solves of
+            // eight 1.10 -> 1.13 ms, of sixteen 1.90 -> 1.95 (alone the same).
+            const bool ahead = lv.s_gather.cnt <= (h->num_sms > 0 ? h->num_sms : 148) || nrb * (int)sizeof(T) <= 16;
+            launch_kx(early(h, ahead && h->step_pdl), k_s_gather<T>, (unsigned)lv.s_gather.cnt, 256, 0, h->stream,
                 h->d_fronts, items + lv.s_gather.off, h->d_grow, h->d_gcon, sb.C, sb.W, sb.R, n, nrhs);
             MF_CUDA(cudaGetLastError());
         }

@@ -105,3 +105,20 @@ def test_queued_passes_equal_single_ones(monkeypatch, ldlt, graphs):
         x = x.cpu().numpy().reshape(3, S.n).T
         assert tm.backward_error(A, x, B.cpu().numpy().reshape(3, S.n).T).max() <= 1e-13
     F.close()
+
+
+@pytest.mark.parametrize("nrhs", [2, 8, 16])
+def test_solves_of_wide_levels_equal_stream_order(monkeypatch, nrhs):
+    """48^3: levels whose forward gather has fewer CTAs than SMs and levels
+    where it has more, with vectors narrow and wide (both launch rules)."""
+    A = tm.grid_laplacian(48, 48, 48, seed=74)
+    P, S = mf.symbolic(A, alg=mf.grid_nd_order(48, 48, 48))
+    B = tm.rhs(S.n, nrhs, seed=15)
+    X = {}
+    for v in ("0", "1"):
+        monkeypatch.setenv("MF_STEP_PDL", v)
+        F = mf.cholesky_(mf.ChordalCholesky(A, P, S))
+        X[v] = mf.ldiv(F, B)
+        F.close()
+    assert np.array_equal(X["0"], X["1"])
+    assert tm.backward_error(A, X["1"], B).max() <= 1e-13
