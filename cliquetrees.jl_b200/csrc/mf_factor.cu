@@ -1137,14 +1137,9 @@ __device__ __forceinline__ void acc_zero(Acc<float>& a) {
         for (int j = 0; j < 4; ++j) a.c[i][j] = 0.f;
 }
 
-template <typename T>
-__device__ __forceinline__ void cp_async_el(T* dst, const T* src, bool valid) {
-    unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
-    int n = valid ? (int)sizeof(T) : 0;
-    if (sizeof(T) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(src), "r"(n));
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(saddr), "l"(src), "r"(n));
+__device__ __forceinline__ void cp_async_el(float* dst, const float* src, bool valid) {
+    const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(saddr), "l"(src), "r"(valid ? 4 : 0));
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -1431,7 +1426,7 @@ __global__ void __launch_bounds__(g64_threads<BM>(), BM == 128 ? 2 : 4) k_gemm64
     const int wr = (warp % (BM / WM)) * WM, wc = (warp / (BM / WM)) * 32;
     const int fr = lane >> 2, fk = lane & 3;
     const double* dj = (LDLT && ROLE != G_TRSM) ? d + f.col0 : nullptr;
-    const bool vec = ((ra | rb) & 1) == 0;
+    const bool vec = BM == 128 || ROLE == G_TRAIL || ((ra | rb) & 1) == 0;  // (even by their lists there)
     const int nchunk = (kend - kbeg + GK - 1) / GK;
     double dn = 0.0;
     if (LDLT && L2 && tid < GK && kbeg + tid < kend) dn = ld_l2(dj + kbeg + tid);

@@ -231,10 +231,10 @@ enum KernelId {
     K_COUNT
 };
 
-// The solves handle a front with one warp when the factorization kept it
-// whole (nj <= kSmallMax) or it is narrow with a short L21 (a warp streams
-// L21 row by row, so a long one serialises); otherwise it is blocked in the
-// factorization too and its diagonal-block inverses exist.
+// Small fronts of the solves (a warp, 16 lanes or a CTA each): the factorization
+// kept it whole (nj <= kSmallMax) or it is narrow with a short L21 (a warp
+// streams L21 row by row, so a long one serialises); other fronts are blocked in
+// the factorization too and their diagonal-block inverses exist.
 constexpr int kSmallSolveNA = 256;
 __host__ __device__ inline bool solve_small(const Front& f) {
     return f.nn + f.na <= kSmallMax || (f.nn <= kNB && f.na <= kSmallSolveNA);

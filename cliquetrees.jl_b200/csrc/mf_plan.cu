@@ -657,8 +657,9 @@ int build_plan(mf_handle* h, const int64_t* resptr, const int64_t* sepptr, const
         end(lv.split_syrk);
         h->nsplit_units = std::max(h->nsplit_units, sunits);
 
-        // solves: small fronts (solve_small) one warp each; blocked fronts in
-        // 256-column super-block steps using the super-block inverses
+        // solves: small fronts (solve_small) a CTA each on levels of at most
+        // kCtaFronts, else a warp or 16 lanes each; blocked fronts in 256-column
+        // super-block steps using the super-block inverses
         int64_t nsmall = 0;
         for (int32_t j : fr) nsmall += solve_small(h->h_fronts[j]) && task_of[j] < 0;
         const bool cta = nsmall <= kCtaFronts;

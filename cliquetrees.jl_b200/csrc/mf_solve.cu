@@ -46,11 +46,11 @@ __global__ void k_diag_div(T* __restrict__ C, const T* __restrict__ d, int64_t n
 }
 
 // ---------------------------------------------------------------------------
-// small fronts (nj <= 96, or nn <= 64 and na <= 256): one warp per front,
-// kSmallWarps fronts per CTA, warp-synchronous (no block barriers).  The
-// front's right-hand-side block C1 (nn x nrhs) lives in the warp's slice of
-// shared memory; lane i holds rows i, i + 32, i + 64 in registers during the
-// triangular solves.
+// small fronts (nj <= 96, or nn <= 64 and na <= 256) of wide levels (narrow
+// levels: mf_solve_small.cu): one warp per front, kSmallWarps fronts per CTA,
+// warp-synchronous (no block barriers).  The front's right-hand-side block C1
+// (nn x nrhs) lives in the warp's slice of shared memory; lane i holds rows i,
+// i + 32, i + 64 in registers during the triangular solves.
 // ---------------------------------------------------------------------------
 constexpr int kSmallWarps = 4;
 constexpr int kSmallRows = (kSmallMax + 31) / 32;  // rows per lane (3)
