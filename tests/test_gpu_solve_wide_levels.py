@@ -3,7 +3,9 @@
 of the single matrix narrow, which the test reads off the plan, so each front
 size is solved both ways.  The operations and their order are the same:
 FP64 solutions must be bitwise equal, with fronts of at most 16, 32 and 96
-rows and of at most 64 columns over a longer separator among them."""
+rows and of at most 64 columns over a longer separator among them.  The
+forest takes its fronts of at most 32 rows 16 or 32 lanes each, and (with
+MF_TINY_SOLVE=0) a warp each like the others."""
 import numpy as np
 import pytest
 
@@ -37,8 +39,10 @@ def small_fronts_by_level(F):
     return [(nn + na)[small & (level == v)] for v in range(info[7])]
 
 
+@pytest.mark.parametrize("tiny", ["1", "0"])
 @pytest.mark.parametrize("ldlt", [False, True])
-def test_every_level_both_ways(ldlt):
+def test_every_level_both_ways(ldlt, tiny, monkeypatch):
+    monkeypatch.setenv("MF_TINY_SOLVE", tiny)
     copies = LIMIT + 6
     A = tm.grid_laplacian(9, 9, 16, seed=83, lo=1e-1, hi=10.0)
     P, S = mf.symbolic(A, alg=mf.grid_nd_order(9, 9, 16))
