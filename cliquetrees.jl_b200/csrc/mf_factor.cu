@@ -1293,10 +1293,11 @@ __global__ void __launch_bounds__(256) k_gemm(const Front* __restrict__ fronts, 
 //     than SMs, which last as long as one tile's products (KKT 24: 12.26 ->
 //     11.75 ms a pass, 100^2 922 -> 886 us).
 // What bounds the large launches is the FP64 pipe (64 FMA a cycle and SM:
-// 36.9 TFLOP/s measured for DMMA alone); 80^3: SYRKs 40.7 -> 36.5 ms, trailing
+// 36.9 TFLOP/s measured for DMMA alone; 87 % active in a large SYRK launch, 79 %
+// in a large trailing update, whose tiles read and write C for 256 of k); 80^3: SYRKs 40.7 -> 36.5 ms, trailing
 // updates 23.1 -> 20.6, left updates 5.9 -> 4.2, KKT 24 left updates 1.56 ->
 // 1.01 ms, against 64 x 64 tiles of eight warps fed by 8-byte copies, two
-// barriers per 32 k. operands come in 16-byte asynchronous copies, three
+// barriers per 32 k.  Operands come in 16-byte asynchronous copies, three
 // stages of 16 k deep, one barrier a stage.  Tiles are columns of the panel
 // (rows contiguous, [k][row] in shared memory with 4 doubles of padding: a
 // fragment read touches every bank once).  A copy needs an even row start;
