@@ -459,7 +459,7 @@ int cuda_fail(cudaError_t e, const char* where);
 //     k_gemm_tc    nothing (barriers and tensor memory are set up)
 //   solves (attribute unless MF_STEP_PDL=0), which write no factor
 //     k_s_cta_fwd, k_s_cta_bwd, k_s_ftile, k_s_btile   panels
-//     k_s_fwd_l, k_s_bwd_l                             panels (early_panel())
+//     k_s_fwd_l, k_s_bwd_l    panels (early_panel(); k_s_bwd_l in single precision)
 //     k_s_sdiag                                        super-block inverses
 //     k_s_gather                                       contribution lists (few CTAs or narrow vectors)
 // k_gemm (LEFT, TRSM), k_s_fwd_red and k_s_bwd_red are launched with the

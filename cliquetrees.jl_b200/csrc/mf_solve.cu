@@ -1928,13 +1928,18 @@ static int solve_impl(mf_handle* h, const SolveBufs<T>& sb, int nrhs) {
         if (!mid && lv.s_bwd_l.cnt) {
             Timer t(h, K_S_BWD_L);
             const unsigned gl = (unsigned)lv.s_bwd_l.cnt;
+            // Early in single precision only (512^2 mixed 8.71 -> 8.55 ms a pass):
+            // in FP64 its CTAs, resident beside the level above, slow that down
+            // (48^3, one right-hand side: 1.12 against 1.36 ms, 0.71 against 0.81 with
+            // three solves overlapping; 58 x 57 x 56 1.53 against 1.96, 1.10 against 1.29).
+            constexpr bool early_l = sizeof(T) == 4;
             const Item* itl = items + lv.s_bwd_l.off;
             switch (nrb) {
-                case 1: launch_kx(early(h, early_panel<T, 1>() && h->step_pdl), k_s_bwd_l<T, 1>, gl, 256, bwd_smem<T, 1>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
-                case 2: launch_kx(early(h, early_panel<T, 2>() && h->step_pdl), k_s_bwd_l<T, 2>, gl, 256, bwd_smem<T, 2>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
-                case 4: launch_kx(early(h, early_panel<T, 4>() && h->step_pdl), k_s_bwd_l<T, 4>, gl, 256, bwd_smem<T, 4>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
-                case 8: launch_kx(early(h, early_panel<T, 8>() && h->step_pdl), k_s_bwd_l<T, 8>, gl, 256, bwd_smem<T, 8>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
-                default: launch_kx(early(h, early_panel<T, 16>() && h->step_pdl), k_s_bwd_l<T, 16>, gl, 256, bwd_smem<T, 16>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 1: launch_kx(early(h, early_l && early_panel<T, 1>() && h->step_pdl), k_s_bwd_l<T, 1>, gl, 256, bwd_smem<T, 1>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 2: launch_kx(early(h, early_l && early_panel<T, 2>() && h->step_pdl), k_s_bwd_l<T, 2>, gl, 256, bwd_smem<T, 2>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 4: launch_kx(early(h, early_l && early_panel<T, 4>() && h->step_pdl), k_s_bwd_l<T, 4>, gl, 256, bwd_smem<T, 4>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                case 8: launch_kx(early(h, early_l && early_panel<T, 8>() && h->step_pdl), k_s_bwd_l<T, 8>, gl, 256, bwd_smem<T, 8>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
+                default: launch_kx(early(h, early_l && early_panel<T, 16>() && h->step_pdl), k_s_bwd_l<T, 16>, gl, 256, bwd_smem<T, 16>(), h->stream, h->d_fronts, itl, h->d_septgt, sb.P, sb.C, sb.part, sb.W, n, nrhs); break;
             }
             MF_CUDA(cudaGetLastError());
             if (lv.s_bwd_red.cnt) launch_kx(early(h, h->step_pdl), k_s_bwd_red<T>, (unsigned)lv.s_bwd_red.cnt, 256, 0, h->stream, h->d_fronts, items + lv.s_bwd_red.off,
